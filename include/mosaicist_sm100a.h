@@ -136,6 +136,39 @@ int msc_grouped_gemm_mxfp8_ragged(const void* a_q, const void* a_sf, const void*
                                   const float* row_scale, void* out, int l, int rows_total,
                                   int n, int k, const msc_gemm_cfg* cfg, void* stream);
 
+/* Added to a quantiser's sf_layout: rows that are not live (at or beyond masked_m, outside every
+ * group, padding of the last 128-row tile) get zero scale bytes; otherwise those are not written. */
+#define MSC_SF_ZERO_REST 2
+
+/* The masked MoE layer in one call: quantise, GEMM1 with SiLU(gate) * up and requantisation
+ * (one kernel when 2n % 256 == 0), GEMM2 - moe_masked of the reference
+ * (experiments/flashinfer-megamoe-sm100a/moe.py:47-79).
+ *   hidden (l, m, k) bf16, m % 128 == 0; w1_q (l, 2n, k/2), w2_q (l, k, n/2) with tiled scales;
+ *   masked_m (l) int32; input_gs, a2_gs (l) fp32.  The GEMMs' factors are g1_alpha / g2_alpha (l)
+ *   where given, else w1_alpha / (input_gs * w1_gs) and w2_alpha / (a2_gs * w2_gs), worked out in
+ *   the GEMMs' epilogues;
+ *   workspace: msc_moe_masked_workspace(l, m, k, n) bytes, 256-byte aligned, contents irrelevant;
+ *   out (l, m, k) bf16; rows at or beyond masked_m are zeroed with zero_rest, else not written. */
+size_t msc_moe_masked_workspace(int l, int m, int k, int n);
+int msc_moe_masked(const void* hidden, const void* w1_q, const void* w1_sf, const float* w1_gs,
+                   const float* w1_alpha, const void* w2_q, const void* w2_sf, const float* w2_gs,
+                   const float* w2_alpha, const int32_t* masked_m, const float* input_gs,
+                   const float* a2_gs, const float* g1_alpha, const float* g2_alpha, void* workspace,
+                   size_t workspace_bytes, void* out, int zero_rest, int l, int m, int k, int n,
+                   void* stream);
+
+/* The general row quantiser; the named entry points below are special cases of it.
+ *   format 0 NVFP4, 1 MXFP8; x_form 0 bf16, 1 fp32, 2 (NVFP4 only) bf16 gate | up of width 2k,
+ *   quantised as silu(gate) * up; global_scale (l) for NVFP4;
+ *   group_offsets (l) ascending multiples of 128 with group_rows (l), or NULL: group g owns rows
+ *   [g * m_stride, + group_rows[g]) (group_rows NULL: all of them);
+ *   zero_out_bf16 (rows_total, k) or NULL: rows that are not live are set to zero there, so a
+ *   caller whose result has the shape of x needs no separate clearing pass. */
+int msc_quantize_rows(int format, const void* x, int x_form, const float* global_scale,
+                      const int32_t* group_offsets, const int32_t* group_rows, void* q, void* sf,
+                      int sf_layout, void* zero_out_bf16, int l, int rows_total, int m_stride, int k,
+                      void* stream);
+
 /* NVFP4 quantisation of activations: q = e2m1, one e4m3 scale per 16 K-elements,
  *   sf = e4m3(clip(amax/6 * gs, 0, 448)),  q = e2m1_rne(clip(x / (f32(sf)/gs), -6, 6)).
  * Replaces quantize_nvfp4 (experiments/flashinfer-megamoe-sm100a/nvfp4.py:39-57) and its

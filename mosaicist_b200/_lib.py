@@ -44,6 +44,9 @@ SIGNATURES = {
     "msc_grouped_gemm_nvfp4_ragged": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _CFG, _P]),
     "msc_grouped_gemm_nvfp4_swiglu_ragged": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _CFG, _P]),
     "msc_grouped_gemm_mxfp8_ragged": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _CFG, _P]),
+    "msc_moe_masked_workspace": (ctypes.c_size_t, [_I, _I, _I, _I]),
+    "msc_moe_masked": (_I, [_P] * 15 + [ctypes.c_size_t, _P, _I, _I, _I, _I, _I, _P]),
+    "msc_quantize_rows": (_I, [_I, _P, _I, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P]),
     "msc_nvfp4_quantize": (_I, [_P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "msc_nvfp4_silu_mul_quantize": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "msc_nvfp4_quantize_ragged": (_I, [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
@@ -90,6 +93,24 @@ def load() -> ctypes.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+def host_ops():
+    """The native host path (host_ops/host_ops.cpp), built on first use where it is missing."""
+    try:
+        from . import _host_ops
+    except ImportError:
+        from . import build
+
+        build.build_host_ops(force=True)
+        from . import _host_ops
+    return _host_ops
+
+
+def addresses() -> dict:
+    """Address of every entry point of the loaded library (for the native host path)."""
+    lib = load()
+    return {name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES}
 
 
 def check(code: int) -> None:

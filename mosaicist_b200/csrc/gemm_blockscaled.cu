@@ -332,7 +332,7 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const bool valid = row_warp + lane < cur.rows;
       const bool whole_warp = row_warp + 32 <= cur.rows;
       const size_t out_row = (size_t)cur.off + row_warp + lane;
-      float scale = p.alpha ? __ldg(p.alpha + cur.g) : 1.0f;
+      float scale = group_alpha(p, cur.g);
       if (p.row_scale && valid) scale *= __ldg(p.row_scale + out_row);
 
       uint32_t v[4][32];
@@ -456,11 +456,10 @@ static int pick_stages(int stages, const CUtensorMap& ta, const CUtensorMap& tb,
 
 // Shared body of the three entry points.  k_bytes: bytes of K per row; chunk_elems: K
 // elements one 512-byte scale chunk covers.
-static int grouped_gemm(int kind, const void* a_q, const void* a_sf, const void* b_q,
-                        const void* b_sf, const float* alpha, const int32_t* group_offsets,
-                        const int32_t* group_rows, const float* row_scale, void* out, int l,
-                        long long rows_total, int m_stride, int n, int k,
-                        const msc_gemm_cfg* cfg_in, void* stream_v) {
+int grouped_gemm(int kind, const void* a_q, const void* a_sf, const void* b_q, const void* b_sf,
+                 const float* alpha, const int32_t* group_offsets, const int32_t* group_rows,
+                 const float* row_scale, void* out, int l, long long rows_total, int m_stride, int n, int k,
+                 const msc_gemm_cfg* cfg_in, void* stream_v, const float* gs_a, const float* gs_b) {
   msc_gemm_cfg cfg = {};
   if (cfg_in) cfg = *cfg_in;
   if (!a_q || !a_sf || !b_q || !b_sf || !out) return fail(MSC_ERR_BAD_ARG, "NULL operand pointer");
@@ -497,10 +496,12 @@ static int grouped_gemm(int kind, const void* a_q, const void* a_sf, const void*
   rc = make_tmap_bf16_2d(&tc, out, (uint64_t)rows_total, (uint64_t)n, 32);
   if (rc) return rc;
 
-  GemmParams p;
+  GemmParams p = {};
   p.sfa = static_cast<const uint8_t*>(a_sf);
   p.sfb = static_cast<const uint8_t*>(b_sf);
   p.alpha = alpha;
+  p.alpha_gs_a = gs_a;
+  p.alpha_gs_b = gs_b;
   p.row_scale = (cfg.epilogue == MSC_EPI_ROW_SCALE) ? row_scale : nullptr;
   p.group_rows = group_rows;
   p.group_offsets = group_offsets;
@@ -605,7 +606,7 @@ int msc_grouped_gemm_nvfp4_swiglu_ragged(const void* a_q, const void* a_sf, cons
     return fail(MSC_ERR_BAD_ARG, "d_q must be 16-byte aligned, d_sf 4-byte aligned");
   int* status = status_word();
   if (!status) return fail(MSC_ERR_CUDA, "status word unavailable on this device");
-  GemmParams p;
+  GemmParams p = {};
   p.sfa = static_cast<const uint8_t*>(a_sf);
   p.sfb = static_cast<const uint8_t*>(w1_sf);
   p.alpha = alpha;
@@ -658,7 +659,7 @@ int msc_grouped_gemm_nvfp4_scatter_ragged(const void* a_q, const void* a_sf, con
     return fail(MSC_ERR_BAD_ARG, "scale pointers must be 16-byte aligned");
   int* status = status_word();
   if (!status) return fail(MSC_ERR_CUDA, "status word unavailable on this device");
-  GemmParams p;
+  GemmParams p = {};
   p.sfa = static_cast<const uint8_t*>(a_sf);
   p.sfb = static_cast<const uint8_t*>(b_sf);
   p.alpha = alpha;

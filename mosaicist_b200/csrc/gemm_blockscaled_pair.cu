@@ -368,7 +368,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const bool valid = row_warp + lane < cur.rows;
       const bool whole_warp = row_warp + 32 <= cur.rows;
       const size_t out_row = (size_t)cur.off + row_warp + lane;
-      float scale = p.alpha ? __ldg(p.alpha + cur.g) : 1.0f;
+      float scale = group_alpha(p, cur.g);
       if (p.row_scale && valid) scale *= __ldg(p.row_scale + out_row);
 
       uint32_t v[4][32];

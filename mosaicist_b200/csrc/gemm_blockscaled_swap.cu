@@ -364,7 +364,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
       if (!ok) break;
       tc_fence_after_sync();
       if (warp == 0) MSC_STAMP(2, tl, 0);
-      const float alpha = p.alpha ? __ldg(p.alpha + cur.g) : 1.0f;
+      const float alpha = group_alpha(p, cur.g);
       const size_t row0 = (size_t)cur.off + (size_t)tt * 256;   // first token row of the tile
       // 32 tokens of this lane's row, as read from TMEM -> alpha (and the tokens' row scales)
       // applied, rounded to bf16, two tokens per register

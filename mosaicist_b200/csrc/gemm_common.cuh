@@ -15,6 +15,8 @@ struct GemmParams {
   const uint8_t* sfa;        // [row_tiles][sf_chunks][512]
   const uint8_t* sfb;        // [l][n/128][sf_chunks][512]
   const float* alpha;        // [l] or null
+  const float* alpha_gs_a;   // [l] or null, with alpha_gs_b: the group's factor is
+  const float* alpha_gs_b;   // alpha / (alpha_gs_a * alpha_gs_b), the two-level scales' fold
   const float* row_scale;    // [rows_total] or null
   const int* group_rows;     // [l] or null (= m_stride)
   const int* group_offsets;  // [l] or null (= g * m_stride)
@@ -62,6 +64,14 @@ extern int g_debug_flags;
 #define MSC_FLAG(bit) false
 #endif
 
+// Factor of a group's accumulators.
+__device__ __forceinline__ float group_alpha(const GemmParams& p, int g) {
+  if (!p.alpha) return 1.0f;
+  const float a = __ldg(p.alpha + g);
+  if (!p.alpha_gs_a) return a;
+  return __fdiv_rn(a, __fmul_rn(__ldg(p.alpha_gs_a + g), __ldg(p.alpha_gs_b + g)));
+}
+
 // Walks the flattened (group, m-tile, n-tile) space in increasing tile id.
 struct TileCursor {
   int g = 0, base = 0, mtiles = 0, rows = 0, off = 0;
@@ -101,6 +111,14 @@ struct TileCursor {
     return true;
   }
 };
+
+// Body of the block-scaled entry points (gemm_blockscaled.cu): k_bytes and chunk size follow from
+// kind; gs_a / gs_b as in GemmParams.
+int grouped_gemm(int kind, const void* a_q, const void* a_sf, const void* b_q, const void* b_sf,
+                 const float* alpha, const int32_t* group_offsets, const int32_t* group_rows,
+                 const float* row_scale, void* out, int l, long long rows_total, int m_stride, int n, int k,
+                 const msc_gemm_cfg* cfg_in, void* stream_v, const float* gs_a = nullptr,
+                 const float* gs_b = nullptr);
 
 // Launcher of the CTA-pair kernel (gemm_blockscaled_pair.cu).
 int launch_pair_gemm(int kind, const void* a_q, const void* b_q, long long rows_total, long long k_bytes,

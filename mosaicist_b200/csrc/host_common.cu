@@ -4,6 +4,8 @@
 #include <dlfcn.h>
 #include <string.h>
 
+#include <atomic>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <set>
@@ -27,17 +29,17 @@ int fail(int code, const char* fmt, ...) {
 __device__ int g_status_word;
 
 int* status_word() {
-  static std::mutex mu;
-  static int* cached[64] = {nullptr};
+  static std::atomic<int*> cached[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!cached[dev]) {
+  int* w = cached[dev].load(std::memory_order_acquire);
+  if (!w) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
-    cached[dev] = static_cast<int*>(p);
+    w = static_cast<int*>(p);
+    cached[dev].store(w, std::memory_order_release);
   }
-  return cached[dev];
+  return w;
 }
 
 int allow_dynamic_smem(const void* kernel, int bytes) {
@@ -70,10 +72,10 @@ EncodeTiledFn encode_tiled_fn() {
 namespace {
 struct TmapKey {
   const void* base;
-  uint64_t rows, row_bytes;
+  uint64_t rows, row_bytes, pitch;
   uint32_t box_rows;  // bits 31-28: 2 bf16 store map, 1 unswizzled scale map, 3 unswizzled 32-byte box, 0 operand map
   bool operator==(const TmapKey& o) const {
-    return base == o.base && rows == o.rows && row_bytes == o.row_bytes && box_rows == o.box_rows;
+    return base == o.base && rows == o.rows && row_bytes == o.row_bytes && pitch == o.pitch && box_rows == o.box_rows;
   }
 };
 struct TmapKeyHash {
@@ -81,79 +83,103 @@ struct TmapKeyHash {
     size_t h = reinterpret_cast<size_t>(k.base) * 0x9E3779B97F4A7C15ull;
     h ^= k.rows + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
     h ^= k.row_bytes + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
+    h ^= k.pitch + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
     return h ^ k.box_rows;
   }
 };
-int encode_tmap_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
+int encode_tmap_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch,
                    uint32_t box_rows, int flavour);
 }  // namespace
 
 // A tensor map only encodes address, shape and box, so one encoded for a buffer stays valid
 // for any later buffer at the same address with the same shape: cache them, the driver call
-// costs microseconds and the GEMM itself runs for about ten.
+// costs microseconds and the GEMM itself runs for about ten.  In front of the shared table every
+// thread has a small direct-mapped one of its own, without a lock (a call looks three to six maps
+// up); clearing the shared table moves the epoch on, which empties the others.
 static std::mutex g_tmap_mu;
 static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> g_tmap_cache;
+static std::atomic<unsigned> g_tmap_epoch{1};
 
 void clear_tmap_cache() {
   std::lock_guard<std::mutex> lock(g_tmap_mu);
   g_tmap_cache.clear();
+  g_tmap_epoch.fetch_add(1);
 }
 
-static int cached_tmap(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
+static int cached_tmap(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch,
                        uint32_t box_rows, int flavour) {
-  std::mutex& mu = g_tmap_mu;
-  auto& cache = g_tmap_cache;
-  const TmapKey key{base, rows, row_bytes, box_rows | ((uint32_t)flavour << 28)};
+  struct Slot {
+    TmapKey key;
+    unsigned epoch;
+    CUtensorMap map;
+  };
+  constexpr size_t kSlots = 128;
+  static thread_local std::unique_ptr<Slot[]> slots;
+  if (!slots) slots.reset(new Slot[kSlots]());
+  const TmapKey key{base, rows, row_bytes, pitch, box_rows | ((uint32_t)flavour << 28)};
+  size_t h = TmapKeyHash()(key);
+  h ^= h >> 29;
+  h *= 0xBF58476D1CE4E5B9ull;
+  Slot& slot = slots[(h >> 40) % kSlots];
+  const unsigned epoch = g_tmap_epoch.load(std::memory_order_acquire);
+  if (slot.epoch == epoch && slot.key == key) {
+    *map = slot.map;
+    return MSC_OK;
+  }
+  bool have = false;
   {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
+    std::lock_guard<std::mutex> lock(g_tmap_mu);
+    auto it = g_tmap_cache.find(key);
+    if (it != g_tmap_cache.end()) {
       *map = it->second;
-      return MSC_OK;
+      have = true;
     }
   }
-  const int rc = encode_tmap_2d(map, base, rows, row_bytes, box_rows, flavour);
-  if (rc == MSC_OK) {
-    std::lock_guard<std::mutex> lock(mu);
-    if (cache.size() > 4096) cache.clear();
-    cache.emplace(key, *map);
+  if (!have) {
+    if (const int rc = encode_tmap_2d(map, base, rows, row_bytes, pitch, box_rows, flavour)) return rc;
+    std::lock_guard<std::mutex> lock(g_tmap_mu);
+    if (g_tmap_cache.size() > 4096) g_tmap_cache.clear();
+    g_tmap_cache.emplace(key, *map);
   }
-  return rc;
+  slot.key = key;
+  slot.map = *map;
+  slot.epoch = epoch;
+  return MSC_OK;
 }
 
 int make_tmap_bytes_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                        uint32_t box_rows) {
-  return cached_tmap(map, base, rows, row_bytes, box_rows, 0);
+  return cached_tmap(map, base, rows, row_bytes, row_bytes, box_rows, 0);
 }
 
 int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                       uint32_t box_rows) {
-  return cached_tmap(map, base, rows, cols * 2, box_rows, 2);
+  return cached_tmap(map, base, rows, cols * 2, cols * 2, box_rows, 2);
 }
 
 int make_tmap_sf_2d(CUtensorMap* map, const void* base, uint64_t rows128, uint32_t box_rows) {
-  return cached_tmap(map, base, rows128, 128, box_rows, 1);
+  return cached_tmap(map, base, rows128, 128, 128, box_rows, 1);
 }
 
 int make_tmap_narrow_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                         uint32_t box_rows) {
-  return cached_tmap(map, base, rows, row_bytes, box_rows, 3);
+  return cached_tmap(map, base, rows, row_bytes, row_bytes, box_rows, 3);
 }
 
 namespace {
-int encode_tmap_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
+int encode_tmap_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch,
                    uint32_t box_rows, int flavour) {
   const bool bf16 = flavour == 2;
   const bool swizzled = flavour == 0 || flavour == 2;
   const cuuint32_t box_bytes = flavour == 3 ? 32u : 128u;
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return MSC_ERR_CUDA;
-  if (reinterpret_cast<uintptr_t>(base) % 16 || row_bytes % 16)
-    return fail(MSC_ERR_BAD_ARG, "operand base and row pitch must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(base) % 16 || row_bytes % 16 || pitch % 16)
+    return fail(MSC_ERR_BAD_ARG, "operand base, row length and row pitch must be 16-byte aligned");
   if (box_rows == 0 || box_rows > 256) return fail(MSC_ERR_BAD_ARG, "box rows out of range");
   // the box is 128 bytes wide (128 byte elements or 64 bf16 elements), 32 for the narrow flavour
   cuuint64_t dims[2] = {bf16 ? row_bytes / 2 : row_bytes, rows};
-  cuuint64_t strides[1] = {row_bytes};
+  cuuint64_t strides[1] = {pitch};
   cuuint32_t box[2] = {bf16 ? 64u : box_bytes, box_rows};
   cuuint32_t estr[2] = {1u, 1u};
   CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
@@ -169,21 +195,7 @@ int encode_tmap_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t r
 
 int make_tmap_pitched_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                          uint64_t pitch_bytes, uint32_t box_rows) {
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) return MSC_ERR_CUDA;
-  if (reinterpret_cast<uintptr_t>(base) % 16 || pitch_bytes % 16 || row_bytes % 16)
-    return fail(MSC_ERR_BAD_ARG, "matrix base, row length and pitch must be 16-byte aligned");
-  if (box_rows == 0 || box_rows > 256) return fail(MSC_ERR_BAD_ARG, "box rows out of range");
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {pitch_bytes};
-  cuuint32_t box[2] = {128u, box_rows};
-  cuuint32_t estr[2] = {1u, 1u};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides,
-                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return fail(MSC_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-  return MSC_OK;
+  return cached_tmap(map, base, rows, row_bytes, pitch_bytes, box_rows, 0);
 }
 
 int num_sms() {

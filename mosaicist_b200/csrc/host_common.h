@@ -61,6 +61,15 @@ int num_sms();
 int launch_sf_swizzle(const void* sf_rowmajor, void* sf_tiled, int groups, int mn, int kwords,
                       const int* rows_used, cudaStream_t stream);
 
+// The row quantisers (quantize.cu, quantize_mx.cu).  group_offsets null: masked layout, group g
+// owns rows [g * m_stride, + group_rows[g]).  sf_layout may carry MSC_SF_ZERO_REST; zero_out: see
+// msc_quantize_rows.
+int quantize_nvfp4_rows(const void* x, int x_dtype, const float* gs, const int32_t* group_offsets,
+                        const int32_t* group_rows, void* q, void* sf, int sf_layout, int l,
+                        long long rows_total, int m_stride, int k, int silu, void* zero_out, void* stream);
+int quantize_mxfp8_rows(const void* x, int x_dtype, const int32_t* group_offsets, const int32_t* group_rows,
+                        void* q, void* sf, int sf_layout, int l, long long rows, int k, void* stream);
+
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device); safe to call from
 // several host threads.
 int allow_dynamic_smem(const void* kernel, int bytes);
