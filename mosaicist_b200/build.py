@@ -46,7 +46,9 @@ def _stale() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
-    """Compile every .cu under csrc/ into one shared library; returns its path."""
+    """Compile every .cu under csrc/ into one shared library (and the native host path beside
+    it); returns its path."""
+    build_host_ops(force)
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not force and not _stale():
         return LIB
@@ -70,6 +72,40 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         if res.returncode != 0:
             raise RuntimeError("nvcc -ptx failed:\n" + res.stderr[-4000:])
     return LIB
+
+
+HOST_OPS_SRC = PKG / "host_ops" / "host_ops.cpp"
+HOST_OPS = PKG / "_host_ops.so"
+
+
+def build_host_ops(force: bool = False) -> pathlib.Path:
+    """The native host path of the operators (host_ops/host_ops.cpp), a Python extension module
+    against torch's C++ interface; returns its path."""
+    deps = [HOST_OPS_SRC, PKG.parent / "include" / "mosaicist_sm100a.h"]
+    if not force and HOST_OPS.exists() and all(p.stat().st_mtime <= HOST_OPS.stat().st_mtime for p in deps):
+        return HOST_OPS
+    gxx = shutil.which("g++")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if gxx is None:
+        if HOST_OPS.exists():
+            return HOST_OPS  # prebuilt module on a machine without a compiler
+        raise RuntimeError("g++ not found and no prebuilt _host_ops.so")
+    import sysconfig
+
+    import torch
+
+    root = pathlib.Path(torch.__file__).resolve().parent
+    cuda = pathlib.Path(nvcc).resolve().parents[1]
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+                sysconfig.get_paths()["include"]]
+    cmd = [gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in includes],
+           "-o", str(HOST_OPS), str(HOST_OPS_SRC), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed on the host operators:\n" + res.stderr[-4000:])
+    return HOST_OPS
 
 
 CUPTI_SHIM = PKG / "cupti_shim" / "libmsc_cupti.so"
@@ -113,6 +149,7 @@ def build_debug(force: bool = False) -> pathlib.Path:
 if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose=True)
     print("built", path)
+    print("built", build_host_ops(force="--force" in sys.argv))
     print("built", build_cupti_shim(force="--force" in sys.argv))
     if "--debug" in sys.argv:
         print("built", build_debug(force="--force" in sys.argv))

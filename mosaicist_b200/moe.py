@@ -18,8 +18,11 @@ import torch
 
 from . import _lib, ops
 
+_host_ops = _lib.host_ops()
+
 
 _OFFSETS = {}
+_DEFAULT_CONFIG = ops.GemmConfig()
 
 
 def _masked_offsets(l: int, m: int, device) -> torch.Tensor:
@@ -37,16 +40,23 @@ def fold_alphas(w1_gs, w1_alpha, w2_gs, w2_alpha, input_global_scale, a2_global_
 
 
 def moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
-               input_global_scale, a2_global_scale, gemm1_config=ops.GemmConfig(),
-               gemm2_config=ops.GemmConfig(), fuse_gemm1: bool | None = None, folded_alphas=None):
+               input_global_scale, a2_global_scale, gemm1_config=_DEFAULT_CONFIG,
+               gemm2_config=_DEFAULT_CONFIG, fuse_gemm1: bool | None = None, folded_alphas=None):
     """(l, m, k) bf16 in, (l, m, k) bf16 out; rows >= masked_m[l] are left untouched.
     Same arguments as the reference's moe_masked: w1_q (l, 2n, k/2), w1_sf / w2_sf in the MMA
     tiling, w2_q (l, k, n/2), per-expert global scales and alphas (l,) f32.
     fuse_gemm1: GEMM1, SiLU(gate) * up and the requantisation run as one kernel, as the
     reference's fused variant does (gemm1_silu_quantize.py:94); bit-identical to the three-kernel
     form.  Default: whenever 2n % 256 == 0 (at the reference's l=8 m=512 k=2048 n=1024 the
-    layer takes 37.0 us fused against 40.0 us as separate kernels).  folded_alphas = fold_alphas(...) skips the four small elementwise kernels that fold
-    the global scales into the GEMM alphas (they only depend on the weights and scales)."""
+    layer takes 37.0 us fused against 40.0 us as separate kernels).  folded_alphas = fold_alphas(...)
+    saves the GEMMs the division that folds the global scales into their alphas.
+
+    With the default configurations the layer is one native call (msc_moe_masked)."""
+    if (fuse_gemm1 is None or fuse_gemm1 == (w1_q.shape[1] % 256 == 0)) and masked_m is not None and \
+            gemm1_config == _DEFAULT_CONFIG and gemm2_config == _DEFAULT_CONFIG:
+        g1_alpha, g2_alpha = folded_alphas if folded_alphas is not None else (None, None)
+        return _host_ops.moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
+                                    input_global_scale, a2_global_scale, g1_alpha, g2_alpha)
     a_q, a_sf = ops.quantize_nvfp4(hidden, input_global_scale, masked_m)
     g1_alpha, g2_alpha = folded_alphas if folded_alphas is not None else fold_alphas(
         w1_gs, w1_alpha, w2_gs, w2_alpha, input_global_scale, a2_global_scale)
@@ -141,11 +151,8 @@ class MegaMoE:
 
     def route(self, logits):
         """logits (T, experts_total) f32 -> fills ids / weights; returns them."""
-        T, experts = logits.shape
-        lib = _lib.load()
-        _lib.check(lib.msc_moe_route_topk(logits.data_ptr(), self.ids.data_ptr(),
-                                          self.weights.data_ptr(), T, experts, self.topk,
-                                          torch.cuda.current_stream().cuda_stream))
+        T = logits.shape[0]
+        _host_ops.moe_route(self, logits)
         return self.ids[:T], self.weights[:T]
 
     def forward(self, tokens, logits=None, out=None):
@@ -154,29 +161,9 @@ class MegaMoE:
         T = tokens.shape[0]
         if T > self.max_tokens:
             raise ValueError(f"{T} tokens exceed the workspace built for {self.max_tokens}")
-        lib = _lib.load()
-        st = torch.cuda.current_stream().cuda_stream
-        if logits is not None:
-            self.route(logits)
-        K, E = self.topk, self.E
-        _lib.check(lib.msc_moe_plan(self.ids.data_ptr(), T * K, self.expert_first, E,
-                                    self.rank.data_ptr(), self.group_rows.data_ptr(),
-                                    self.group_offsets.data_ptr(), self.total_rows.data_ptr(),
-                                    self.scratch.data_ptr(), st))
-        _lib.check(lib.msc_moe_permute_quantize(
-            tokens.data_ptr(), self.ids.data_ptr(), self.weights.data_ptr(), self.rank.data_ptr(),
-            self.group_offsets.data_ptr(), self.input_gs.data_ptr(), T, self.h, K,
-            self.expert_first, E, self.a_q.data_ptr(), self.a_sf.data_ptr(),
-            self.row_weight.data_ptr(), self.row_token.data_ptr(),
-            None if self.sf_rows is None else self.sf_rows.data_ptr(), self.rows_cap,
-            self.total_rows.data_ptr(), st))
+        _host_ops.moe_dispatch(self, tokens, logits)
         self.run_experts()
-        if out is None:
-            out = torch.empty((T, self.h), dtype=torch.bfloat16, device=tokens.device)
-        _lib.check(lib.msc_moe_unpermute(self.y.data_ptr(), self.ids.data_ptr(), self.rank.data_ptr(),
-                                         self.group_offsets.data_ptr(), out.data_ptr(), T, self.h, K,
-                                         self.expert_first, E, st))
-        return out
+        return _host_ops.moe_combine(self, tokens, out)
 
     def run_experts(self):
         """GEMM1 -> SiLU*up + quantise -> GEMM2 over the grouped rows in a_q / a_sf (layout in
