@@ -25,7 +25,8 @@ PTX = PKG / "libmosaicist_sm100a.ptx"
 #: msc_ptx_path() points, the others beside it with a suffix
 PTX_UNITS = {"pair": ("gemm_blockscaled_pair.cu", PTX),
              "single": ("gemm_blockscaled.cu", PKG / "libmosaicist_sm100a.single.ptx"),
-             "dense": ("gemm_dense_f16.cu", PKG / "libmosaicist_sm100a.dense.ptx")}
+             "dense": ("gemm_dense_f16.cu", PKG / "libmosaicist_sm100a.dense.ptx"),
+             "int4": ("gemm_int4.cu", PKG / "libmosaicist_sm100a.int4.ptx")}
 PTXAS_LOG = PKG / "libmosaicist_sm100a.ptxas.log"
 DEBUG_LIB = PKG / "libmosaicist_sm100a_debug.so"
 
@@ -57,7 +58,7 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
             return LIB  # prebuilt library on a machine without the toolkit
         raise RuntimeError("nvcc not found and no prebuilt libmosaicist_sm100a.so")
     srcs = [str(s) for s in sources()]
-    cmd = [nvcc, *ARCH, *COMMON, "-Xptxas", "-v", "-shared", "-Xcompiler", "-fPIC",
+    cmd = [nvcc, *ARCH, *COMMON, "-Xptxas", "-v", "-t", "0", "-shared", "-Xcompiler", "-fPIC",
            "-cudart", "static", "-o", str(LIB), *srcs, "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     PTXAS_LOG.write_text(res.stderr)

@@ -105,7 +105,31 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
-// The same wait made by all 32 lanes of a converged warp, with a warp-uniform result.
+// The same wait for a warp that others do not wait for (a producer ahead of its consumers, an
+// epilogue during a long main loop): it sleeps between probes, so that its polling does not take
+// issue slots from warps that compute.
+__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                                  int* status, int code, uint32_t sleep_ns) {
+  if (mbar_test(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (true) {
+    __nanosleep(sleep_ns);
+    if (mbar_test(bar, parity)) return true;
+    if (*abort_flag) return false;
+    if (clock64() - t0 > kWaitBudgetCycles) {
+      *abort_flag = 1u;
+      if (status) atomicCAS(status, 0, kStatusTimeout | code);
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ bool warp_wait_relaxed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                                  int* status, int code, uint32_t sleep_ns) {
+  const bool ok = mbar_wait_relaxed(bar, parity, abort_flag, status, code, sleep_ns);
+  return __all_sync(0xffffffffu, ok);
+}
+
+// The bounded wait made by all 32 lanes of a converged warp, with a warp-uniform result.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity,
                                           volatile uint32_t* abort_flag, int* status, int code) {
   const bool ok = mbar_wait_bounded(bar, parity, abort_flag, status, code);
@@ -377,6 +401,30 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t adesc,
       " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same with the A operand in tensor memory: lane = row of M, two bf16 of K per 32-bit column.
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      " .reg .pred p;\n"
+      " setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+                                                   uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      " .reg .pred p;\n"
+      " setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 

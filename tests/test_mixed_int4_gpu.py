@@ -124,3 +124,33 @@ def test_fused_int4_kernel_equals_the_two_launch_path(gsz, k):
     assert _lib.status_word() == 0
     assert torch.equal(one.view(torch.int16), two.view(torch.int16))       # NaN rows compare as bits
     assert int(torch.isnan(one).sum()) == (tot - sum(rows_list)) * n
+
+
+@pytest.mark.parametrize("rows_list,n,k,gsz", [
+    # single CTAs (groups within one 128-row block): token edges, 64 K, an odd number of 64-K blocks
+    ([1, 16, 17, 128, 33], 256, 64, 64), ([5, 0, 100], 512, 320, 64), ([15, 32], 256, 1152, 384),
+    # CTA pairs (enough tiles for the machine): rows split over several tiles, a last tile of one row
+    ([300, 0, 129, 16, 257, 512], 2048, 320, 64), ([513, 256, 31, 1, 255, 290], 2048, 896, 128)])
+def test_fused_int4_tile_edges_exact(rows_list, n, k, gsz):
+    from mosaicist_b200 import _lib, ops
+
+    l = len(rows_list)
+    offs, tot = _layout(rows_list)
+    rng = np.random.default_rng([l, n, k, gsz])
+    a = rng.integers(-2, 3, (tot, k)).astype(np.float32).astype(ml_dtypes.bfloat16)
+    q = rng.integers(-8, 8, (l, n, k)).astype(np.int8)
+    sc = (rng.integers(1, 5, (l, n, k // gsz)).astype(np.float32) / 4).astype(ml_dtypes.bfloat16)
+    out = torch.full((tot, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.mixed_grouped_gemm_int4(_bf16_t(a), T(X.pack_int4(q)), _bf16_t(sc), T(np.array(offs, np.int32)),
+                                T(np.array(rows_list, np.int32)), None, gsz, out=out, fused=True)
+    assert _lib.status_word() == 0
+    want = X.ragged_gemm_f64(a, X.dequant(q, sc, gsz), offs, rows_list)
+    # the weights are multiples of 1/4 of at most 8, the partial sums multiples of 1/4 below 2^15:
+    # exact in fp32, one rounding to bf16 at the end
+    assert np.abs(want).max() < 2 ** 15 and np.array_equal(want * 4, np.round(want * 4))
+    got = out.float().cpu().numpy()
+    mask = np.zeros((tot, 1), bool)
+    for o, r in zip(offs, rows_list):
+        mask[o:o + r] = True
+    assert np.array_equal(np.where(mask, got, 0), O.bf16_round(want))
+    assert np.isnan(got[~mask[:, 0]]).all()
