@@ -239,10 +239,19 @@ int msc_sf_swizzle(const void* sf_rowmajor, void* sf_tiled, int groups, int mn, 
  * multi-GPU form) is the shard's base pointer with the parent's pitch.  k, n and the pitches
  * must be multiples of 8; m, n, k need not be tile multiples.  max_ctas 0 = one CTA per SM.
  * Problems with enough columns run 256 x 512 tiles (two MMAs per K step share the A stage, so
- * the kernel is bounded by the tensor pipe rather than by L2 -> SM traffic); a negative max_ctas
- * forces the 256 x 256 form on |max_ctas| CTAs. */
+ * the kernel is bounded by the tensor pipe rather than by L2 -> SM traffic), problems with too few
+ * of them one 128-row tile per cluster (max_ctas = 0 only); a negative max_ctas forces the
+ * 256 x 256 form on |max_ctas| CTAs.  All forms add up in the same order, except that with m <= 128
+ * and k >= 4096 the contraction is summed as two halves, whatever n is. */
 int msc_gemm_f16(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb,
                  int ldc, int dtype, int max_ctas, void* stream);
+
+/* msc_gemm_f16 with the tile form chosen by the caller instead of by size.  splits = 0: the
+ * persistent kernel.  splits = 1 .. 8: one tile of 128 rows x tile_n (64 or 128) columns per
+ * cluster, its 64-element K stages (at least one each) dealt out to `splits` CTAs and the parts
+ * summed in fp32 in that order. */
+int msc_gemm_f16_form(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb,
+                      int ldc, int dtype, int tile_n, int splits, void* stream);
 
 /* Mixed-dtype grouped GEMM (bf16 activations x int4 weights with bf16 group scales), as two
  * launches.  Semantics of the reference's port of CUTLASS example 69

@@ -55,6 +55,7 @@ SIGNATURES = {
     "msc_mxfp8_quantize": (_I, [_P, _I, _P, _P, _I, _I, _I, _P]),
     "msc_mxfp8_quantize_ragged": (_I, [_P, _I, _P, _P, _P, _P, _I, _I, _I, _P]),
     "msc_gemm_f16": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
+    "msc_gemm_f16_form": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
     "msc_int4_dequant_bf16": (_I, [_P, _P, _P, _I, _I, _I, _I, _P]),
     "msc_grouped_gemm_bf16_ragged": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
     "msc_grouped_gemm_bf16_int4_ragged": (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),

@@ -29,7 +29,7 @@
 // int4_dequant_kernel (convert to bf16, multiply by the group scale in bf16 — the order the
 // reference prescribes, ports/hopper_mixed_dtype_grouped_gemm/problems.py:75-81) and then
 // multiplied here with fp32 accumulation (problems.py:84-87).
-#include "gemm_common.cuh"
+#include "gemm_dense.h"
 
 #include <cuda_fp16.h>
 
@@ -456,9 +456,9 @@ extern "C" int msc_grouped_gemm_bf16_ragged(const void* a, const void* b, const 
   return MSC_OK;
 }
 
-extern "C" int msc_gemm_f16(const void* a, const void* b, void* c, int m, int n, int k, int lda,
-                            int ldb, int ldc, int dtype, int max_ctas, void* stream) {
-  using namespace msc;
+namespace msc {
+static int dense_gemm(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc, int dtype,
+                      int max_ctas, const DenseForm* forced, void* stream) {
   if (!a || !b || !c) return fail(MSC_ERR_BAD_ARG, "NULL pointer");
   if (m <= 0 || n <= 0 || k <= 0) return fail(MSC_ERR_BAD_ARG, "m, n, k must be positive");
   if (dtype != 0 && dtype != 1) return fail(MSC_ERR_UNSUPPORTED, "dtype must be 0 (fp16) or 1 (bf16)");
@@ -474,6 +474,9 @@ extern "C" int msc_gemm_f16(const void* a, const void* b, void* c, int m, int n,
   if (rc) return rc;
   rc = make_tmap_pitched_2d(&tc, c, (uint64_t)m, (uint64_t)n * 2, (uint64_t)ldc * 2, 32);
   if (rc) return rc;
+  const DenseForm form = forced ? *forced : max_ctas == 0 ? pick_dense_form(m, n, k, lda, ldb) : DenseForm{0, 0};
+  if (form.splits)
+    return launch_dense_split(form, a, b, c, m, n, k, lda, ldb, ldc, dtype, status, static_cast<cudaStream_t>(stream));
   DenseParams p;
   p.m_tiles = (m + 255) / 256;
   p.n_tiles = (n + 255) / 256;
@@ -514,4 +517,16 @@ extern "C" int msc_gemm_f16(const void* a, const void* b, void* c, int m, int n,
       pdl_launch_config(2 * pairs, L::kThreads, L::kAlloc, static_cast<cudaStream_t>(stream), attr);
   MSC_CUDA_OK(cudaLaunchKernelEx(&lc, kern, ta, tb, tc, p));
   return MSC_OK;
+}
+}  // namespace msc
+
+extern "C" int msc_gemm_f16(const void* a, const void* b, void* c, int m, int n, int k, int lda,
+                            int ldb, int ldc, int dtype, int max_ctas, void* stream) {
+  return msc::dense_gemm(a, b, c, m, n, k, lda, ldb, ldc, dtype, max_ctas, nullptr, stream);
+}
+
+extern "C" int msc_gemm_f16_form(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc,
+                                 int dtype, int tile_n, int splits, void* stream) {
+  const msc::DenseForm form{tile_n, splits};
+  return msc::dense_gemm(a, b, c, m, n, k, lda, ldb, ldc, dtype, 0, &form, stream);
 }

@@ -95,3 +95,34 @@ def test_dense_random_and_column_shards(dtype, rel):
         ops.gemm_f16(a, b[:, cols], out=out2[:, cols])
     assert _lib.status_word() == 0
     assert torch.equal(out, out2)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (7, 64, 64), (100, 72, 40), (128, 128, 512), (129, 200, 136),
+                                   (300, 136, 576), (333, 520, 1544)])
+@pytest.mark.parametrize("tile_n,splits", [(64, 1), (64, 2), (64, 8), (128, 1), (128, 3), (128, 4)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_dense_split_forms_exact(m, n, k, tile_n, splits, dtype):
+    """One tile per cluster with the contraction split over its CTAs (msc_gemm_f16_form): exact on
+    integer operands at the edges of tiles and of K stages, inside a wider output whose other columns
+    stay untouched; more splits than K stages are refused."""
+    from mosaicist_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randint(-1, 2, (m, k), device="cuda", generator=g).to(dtype)
+    b = torch.randint(-1, 2, (k, n), device="cuda", generator=g).to(dtype)
+    if k > 512:
+        a = a * (torch.rand((m, k), device="cuda", generator=g) < 0.1).to(dtype)
+    out = torch.full((m, n + 8), -7.0, dtype=dtype, device="cuda")
+    rc = _lib.load().msc_gemm_f16_form(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, k, n, n + 8,
+                                       int(dtype == torch.bfloat16), tile_n, splits,
+                                       torch.cuda.current_stream().cuda_stream)
+    if splits > (k + 63) // 64:
+        assert rc != 0
+        return
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert _lib.status_word() == 0
+    ref = a.double() @ b.double()
+    assert ref.abs().max() <= 256                       # exact in bf16
+    assert torch.equal(out[:, :n].double(), ref)
+    assert torch.all(out[:, n:] == -7.0)
