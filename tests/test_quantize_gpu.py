@@ -226,3 +226,21 @@ def test_mxfp8_quantiser_feeds_the_gemm():
     for o, r in zip(offs, rows_list):
         ok, worst = O.tolerance_ok(got[o:o + r], ref[o:o + r])
         assert ok, worst
+
+
+@pytest.mark.parametrize("per_group", [8, 4096, 8192, 8200, 3 * 8192 + 64, 64 * 8192 + 8])
+@pytest.mark.parametrize("l", [1, 3, 40])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_global_scale_exact_at_piece_edges(per_group, l, dtype):
+    """The maximum may sit in the first or last vector of a group whose size is not a whole number of
+    the kernel's pieces; a NaN does not count."""
+    from mosaicist_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(per_group + l)
+    x = torch.randn((l, per_group), device="cuda", generator=g).to(dtype)
+    for i in range(l):
+        x[i, (0, per_group - 1, per_group // 2)[i % 3]] = -(10.0 + i)
+    x[0, 1] = float("nan")
+    amax = x.abs().float().nan_to_num(0.0).amax(1)
+    want = torch.full_like(amax, 2688.0) / amax
+    assert torch.equal(ops.global_scale_for(x), want)
