@@ -29,19 +29,18 @@
 
 namespace msc {
 
-template <int KIND, int STAGES, bool SWIGLU>
+// A ring stage: 128 weight rows, up to 160 tokens (this CTA's half of a tile's 320), the scales of the
+// weight rows and of up to 384 tokens, in that order.  What a stage holds follows from the largest
+// group of the call, so a decode step gets a deeper ring out of the same shared memory.
+template <int KIND, bool SWIGLU>
 struct SwapSmem {
   static constexpr int kChunks = (KIND == KIND_NVFP4) ? 4 : 1;   // 512-byte scale chunks per 128-row block and stage
-  static constexpr int kHeader = 1024;
   static constexpr int kW = 128 * 128;        // this CTA's 128 weight rows
-  static constexpr int kT = 160 * 128;        // this CTA's half of the tile's (up to) 320 tokens
-  static constexpr int kSfw = kChunks * 512;
-  static constexpr int kSft = 3 * kChunks * 512;    // scales of all (up to) 384 token rows
-  static constexpr int kOffW = kHeader;
-  static constexpr int kOffT = kOffW + STAGES * kW;
-  static constexpr int kOffSfw = kOffT + STAGES * kT;
-  static constexpr int kOffSft = kOffSfw + STAGES * kSfw;
-  static constexpr int kOffC = kOffSft + STAGES * kSft;
+  static constexpr int kSf = kChunks * 512;   // scales of 128 rows
+  static constexpr int kRing = 4 * (kW + 160 * 128 + 4 * kSf);
+  static constexpr int kMaxStages = 8;
+  static constexpr int kOffRing = 1024;
+  static constexpr int kOffC = kOffRing + kRing;
   static constexpr int kEpiWarps = 8;
   static constexpr int kThreads = (kEpiWarps + 2) * 32;
   // SwiGLU: two buffers of 64 tokens x 128 bf16 at a 272-byte pitch (16-byte reads of
@@ -56,6 +55,23 @@ struct SwapSmem {
   static_assert(kAlloc <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
 };
 
+// The ring a call runs: groups of up to 64, 128 or any number of tokens.  Weights stream from HBM in a
+// decode step, and what a CTA keeps in flight decides the rate: 7 stages of 24 KB instead of 4 of 44.
+struct SwapRing {
+  int t_bytes;    // tokens of a CTA
+  int stage;      // bytes of a stage, a multiple of 1024
+  int stages;
+  template <class L>
+  static __device__ __forceinline__ SwapRing make(int max_rows) {
+    SwapRing r;
+    r.t_bytes = max_rows <= 64 ? 32 * 128 : max_rows <= 128 ? 64 * 128 : 160 * 128;
+    const int blocks = max_rows <= 128 ? 1 : 3;                 // 128-token scale blocks
+    r.stage = (L::kW + r.t_bytes + (1 + blocks) * L::kSf + 1023) & ~1023;
+    r.stages = min(L::kRing / r.stage, L::kMaxStages);
+    return r;
+  }
+};
+
 // Token tiles of a group: 256 rows each, the last one also taking a remainder of up to 64.
 __device__ __forceinline__ int swap_token_tiles(int rows) {
   if (rows <= 0) return 0;
@@ -65,29 +81,18 @@ __device__ __forceinline__ int swap_token_tiles(int rows) {
 }
 
 // Walks (group, token tile, weight tile) in increasing tile id; weight tiles vary fastest.
+template <bool KEEP = true>
 struct SwapCursor {
-  int g = 0, base = 0, ttiles = 0, rows = 0, off = 0;
-  bool primed = false;
+  int g = 0, ttiles = 0, rows = 0, off = 0;
+  GroupWindow<KEEP> win;
   __device__ __forceinline__ bool seek(const GemmParams& p, int ntiles, int t, int& tt, int& nt) {
-    while (true) {
-      if (!primed) {
-        if (g >= p.l) return false;
-        rows = __shfl_sync(0xffffffffu, __ldg(p.group_rows + g), 0);
-        off = __shfl_sync(0xffffffffu, __ldg(p.group_offsets + g), 0);
-        if (rows < 0) rows = 0;
-        // a group table that reaches beyond the buffers is cut to what the buffers hold
-        if (off < 0 || off >= p.rows_total) rows = 0;
-        else if (rows > p.rows_total - off) rows = p.rows_total - off;
-        ttiles = swap_token_tiles(rows);
-        primed = true;
-      }
-      const int tiles = ttiles * ntiles;
-      if (t < base + tiles) break;
-      base += tiles;
-      ++g;
-      primed = false;
-    }
-    const int u = t - base;
+    int first;
+    if (!win.find(p.l, t,
+                  [&](int gi, int& r, int& o) { load_group(p.group_rows, p.group_offsets, p.rows_total, gi, r, o); },
+                  [=](int r) { return swap_token_tiles(r) * ntiles; }, g, rows, off, first))
+      return false;
+    ttiles = swap_token_tiles(rows);
+    const int u = t - first;
     tt = u / ntiles;
     nt = u - tt * ntiles;
     return true;
@@ -106,23 +111,24 @@ struct SwapCursor {
   }
 };
 
-template <int KIND, int STAGES, bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SwapSmem<KIND, STAGES, SWIGLU>::kThreads, 1)
+template <int KIND, bool SWIGLU>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SwapSmem<KIND, SWIGLU>::kThreads, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
                  const __grid_constant__ CUtensorMap tmap_t,
                  const __grid_constant__ CUtensorMap tmap_t32,
                  const __grid_constant__ CUtensorMap tmap_sfw,
                  const __grid_constant__ CUtensorMap tmap_sft, const GemmParams p) {
-  using L = SwapSmem<KIND, STAGES, SWIGLU>;
+  using L = SwapSmem<KIND, SWIGLU>;
   static_assert(KIND == KIND_NVFP4 || !SWIGLU, "the fused epilogue quantises to NVFP4");
   constexpr int kChunks = L::kChunks;
   constexpr int kMmaWarp = L::kEpiWarps;
   constexpr int kProducerWarp = L::kEpiWarps + 1;
-  constexpr int kAcc1Col = 128;                 // second accumulator: tokens 128 .. 319
+  constexpr int kAcc1Col = 128;                 // second MMA of a tile: tokens 128 .. 319
+  constexpr int kAccCol = 160;                  // tiles of up to 160 tokens: two accumulators in turn
   // a slot: weights 4 columns per chunk, tokens of the first MMA 8, of the second 8
   constexpr int kSfCol0 = 320, kSlotCols = 20 * kChunks, kSlots = 2;
   constexpr int kSfwCols = 0, kSft0Cols = 4 * kChunks, kSft1Cols = 12 * kChunks;   // offsets inside a slot
-  constexpr uint32_t kSfBoxBytes = kChunks * 512;
+  constexpr uint32_t kSfBoxBytes = L::kSf;
   constexpr uint32_t kIdescBase = (KIND == KIND_NVFP4) ? ((1u << 7) | (1u << 10) | (16u << 24))
                                                        : ((1u << 23) | (16u << 24));
 
@@ -131,10 +137,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const uint32_t sbase = (raw + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - raw);
 
-  const uint32_t bar_full = sbase;                    // STAGES x 8 (used in the leader)
-  const uint32_t bar_empty = sbase + 8 * STAGES;      // STAGES x 8
-  const uint32_t bar_acc_full = sbase + 16 * STAGES;  // 8
-  const uint32_t bar_acc_empty = bar_acc_full + 8;    // 8 (used in the leader)
+  const uint32_t bar_full = sbase;                           // kMaxStages x 8 (used in the leader)
+  const uint32_t bar_empty = sbase + 8 * L::kMaxStages;      // kMaxStages x 8
+  const uint32_t bar_acc_full = sbase + 16 * L::kMaxStages;  // 2 x 8
+  const uint32_t bar_acc_empty = bar_acc_full + 16;          // 2 x 8 (used in the leader)
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sgen + 512);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(sgen + 516);
 
@@ -147,12 +153,14 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const int ntiles = p.n >> 8;   // weight tiles of 256 rows
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < L::kMaxStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
-    mbar_init(bar_acc_full, 1);
-    mbar_init(bar_acc_empty, 2 * L::kEpiWarps);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_acc_full + 8 * b, 1);
+      mbar_init(bar_acc_empty + 8 * b, 2 * L::kEpiWarps);
+    }
     *abort_flag = 0u;
     fence_barrier_init();
   }
@@ -178,9 +186,17 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
   if (p.trace && threadIdx.x == 0) p.trace[(size_t)gridDim.x * 48 + blockIdx.x * 2] = clock64();
 #endif
 
+  // the largest group decides the depth of the ring and whether two accumulators fit; every role of
+  // both CTAs reads the same table
+  int most = 0;
+  for (int g = lane; g < p.l; g += 32) most = max(most, __ldg(p.group_rows + g));
+  most = __reduce_max_sync(0xffffffffu, most);
+  const SwapRing ring = SwapRing::make<L>(most);
+  const bool two_acc = most <= kAccCol;
+
   if (warp == kProducerWarp) {
     // ------------------------------ producer (both CTAs) ------------------------
-    SwapCursor cur;
+    SwapCursor<> cur;
     uint32_t bits = 0;  // per-stage use parity
     bool ok = true;
     uint32_t s = 0;
@@ -209,8 +225,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
         const int c4 = kb * kChunks * 4;
         if (elect_one()) {
           if (leader) mbar_arrive_expect_tx(full, 2 * bytes);
-          tma_load_2d_pair(sbase + L::kOffW + s * L::kW, &tmap_w, full, kb * 128, wrow0);
-          const uint32_t t_dst = sbase + L::kOffT + s * L::kT;
+          const uint32_t w_dst = sbase + L::kOffRing + s * ring.stage;
+          const uint32_t t_dst = w_dst + L::kW, sfw_dst = t_dst + ring.t_bytes;
+          tma_load_2d_pair(w_dst, &tmap_w, full, kb * 128, wrow0);
           if (boxes0 == 4) {
             tma_load_2d_pair(t_dst, &tmap_t, full, kb * 128, trow0);
           } else {
@@ -219,27 +236,27 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
           }
           for (int i = 0; i < boxes1; ++i)   // behind the 64 rows of the first MMA
             tma_load_2d_pair(t_dst + 8192 + i * 4096, &tmap_t32, full, kb * 128, trow1 + 32 * i);
-          tma_load_2d_pair(sbase + L::kOffSfw + s * L::kSfw, &tmap_sfw, full, 0, sfw_row + c4);
-          const uint32_t sft_dst = sbase + L::kOffSft + s * L::kSft;
+          tma_load_2d_pair(sfw_dst, &tmap_sfw, full, 0, sfw_row + c4);
+          const uint32_t sft_dst = sfw_dst + L::kSf;
           for (int bl = 0; bl < blocks; ++bl)
             tma_load_2d_pair(sft_dst + bl * kSfBoxBytes, &tmap_sft, full, 0, sft_row + bl * p.sf_chunks * 4 + c4);
         }
         __syncwarp();
-        s = (s + 1 == STAGES) ? 0u : s + 1;
+        s = (s + 1 == (uint32_t)ring.stages) ? 0u : s + 1;
       }
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer (leader only) --------------------
     if (leader) {
-      SwapCursor cur;
+      SwapCursor<> cur;
       uint32_t bits = 0;
       int tl = 0;
       bool ok = true;
       uint32_t s = 0, slot = 0;
-      const uint64_t wdesc0 = operand_desc_sw128(sbase + L::kOffW);
-      const uint64_t tdesc0 = operand_desc_sw128(sbase + L::kOffT);
-      const uint64_t sfw_d0 = scale_desc(sbase + L::kOffSfw);
-      const uint64_t sft_d0 = scale_desc(sbase + L::kOffSft);
+      const uint64_t wdesc0 = operand_desc_sw128(sbase + L::kOffRing);
+      const uint64_t tdesc0 = operand_desc_sw128(sbase + L::kOffRing + L::kW);
+      const uint64_t sfw_d0 = scale_desc(sbase + L::kOffRing + L::kW + ring.t_bytes);
+      const uint64_t sft_d0 = scale_desc(sbase + L::kOffRing + L::kW + ring.t_bytes + L::kSf);
       for (int t = pair; ok; t += npairs, ++tl) {
         int tt, nt;
         if (!cur.seek(p, ntiles, t, tt, nt)) break;
@@ -247,7 +264,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
         cur.widths(tt, tn, n0, n1);
         const uint32_t idesc0 = kIdescBase | (uint32_t(n0 >> 3) << 17);
         const uint32_t idesc1 = kIdescBase | (uint32_t(n1 >> 3) << 17);
-        ok = warp_wait(bar_acc_empty, (uint32_t)(tl & 1) ^ 1u, abort_flag, p.status, 2);
+        const int buf = two_acc ? (tl & 1) : 0;
+        const uint32_t use = two_acc ? (uint32_t)(tl >> 1) : (uint32_t)tl;
+        const uint32_t acc = tmem_base + buf * kAccCol;
+        ok = warp_wait(bar_acc_empty + 8 * buf, (use & 1u) ^ 1u, abort_flag, p.status, 2);
         if (!ok) break;
         tc_fence_after_sync();
         MSC_STAMP(1, tl, 0);
@@ -263,10 +283,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
           // descriptor low words count 16-byte units: +32 per 512-byte scale chunk, +kBlk per
           // block of 128 rows, +2 per 32 bytes of K in the operand tile, +512 per 64 operand rows
           constexpr int kBlk = kChunks * 32;
-          const uint64_t sfw_d = sfw_d0 + s * (L::kSfw >> 4);
-          const uint64_t sft_d = sft_d0 + s * (L::kSft >> 4);
-          const uint64_t wdesc = wdesc0 + s * (L::kW >> 4);
-          const uint64_t tdesc = tdesc0 + s * (L::kT >> 4);
+          const uint32_t at = s * ((uint32_t)ring.stage >> 4);
+          const uint64_t sfw_d = sfw_d0 + at, sft_d = sft_d0 + at;
+          const uint64_t wdesc = wdesc0 + at, tdesc = tdesc0 + at;
           if (elect_one()) {
 #pragma unroll
             for (int c = 0; c < kChunks; ++c) {
@@ -289,10 +308,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
               if (j < nmma) {
                 const uint32_t accumulate = (j > 0 || kb > 0) ? 1u : 0u;
                 if (KIND == KIND_NVFP4)
-                  tc_mma_nvfp4_pair(tmem_base, wdesc + 2 * j, tdesc + 2 * j, idesc0, sfw_t + 4 * j,
+                  tc_mma_nvfp4_pair(acc, wdesc + 2 * j, tdesc + 2 * j, idesc0, sfw_t + 4 * j,
                                     sft0_t + 8 * j, accumulate);
                 else
-                  tc_mma_mxf8_pair(tmem_base, wdesc + 2 * j, tdesc + 2 * j,
+                  tc_mma_mxf8_pair(acc, wdesc + 2 * j, tdesc + 2 * j,
                                    idesc0 | (uint32_t(j) << 29) | (uint32_t(j) << 4), sfw_t, sft0_t, accumulate);
               }
             }
@@ -313,10 +332,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
             tc_commit_pair(bar_empty + 8 * s, 3);  // frees this stage in both CTAs
           }
           __syncwarp();
-          s = (s + 1 == STAGES) ? 0u : s + 1;
+          s = (s + 1 == (uint32_t)ring.stages) ? 0u : s + 1;
           slot = (slot + 1 == kSlots) ? 0u : slot + 1;
         }
-        if (ok && elect_one()) tc_commit_pair(bar_acc_full, 3);
+        if (ok && elect_one()) tc_commit_pair(bar_acc_full + 8 * buf, 3);
         __syncwarp();
         MSC_STAMP(1, tl, 1);
       }
@@ -325,7 +344,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
     // ------------------------------ epilogue (both CTAs) ------------------------
     // warp w reads lane quadrant w % 4 (32 weight rows = 32 output columns); the two halves
     // w / 4 split the tokens.
-    SwapCursor cur;
+    SwapCursor<!SWIGLU> cur;   // (the plain epilogue sets the pace of short contractions)
     int tl = 0;
     int pass_no = 0;   // SwiGLU: passes so far, over all tiles (selects the staging buffer)
     const int quad = warp & 3;
@@ -342,10 +361,13 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
         const int tok = (2 * i + half) * 32 + lane;
-        rsv[i] = (p.row_scale && tok < tn) ? __ldg(p.row_scale + (size_t)cur.off + (size_t)tt * 256 + tok) : 1.0f;
+        rsv[i] = (!SWIGLU && p.row_scale && tok < tn) ? __ldg(p.row_scale + (size_t)cur.off + (size_t)tt * 256 + tok) : 1.0f;
       }
       bool ok = true;
-      if (lane == 0) ok = mbar_wait_bounded(bar_acc_full, tl & 1, abort_flag, p.status, 4);
+      const int buf = two_acc ? (tl & 1) : 0;
+      const uint32_t use = two_acc ? (uint32_t)(tl >> 1) : (uint32_t)tl;
+      const uint32_t acc = tmem_base + lane_base + buf * kAccCol;
+      if (lane == 0) ok = mbar_wait_bounded(bar_acc_full + 8 * buf, use & 1u, abort_flag, p.status, 4);
       ok = __all_sync(0xffffffffu, ok);
       if (SWIGLU) {
         // the passes below meet at a named barrier: all eight warps go on or none does, or a
@@ -372,7 +394,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float s0 = alpha, s1 = alpha;
-          if (p.row_scale) {
+          if (!SWIGLU && p.row_scale) {
             s0 *= __shfl_sync(0xffffffffu, rs_lane, 2 * i);
             s1 *= __shfl_sync(0xffffffffu, rs_lane, 2 * i + 1);
           }
@@ -393,18 +415,18 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
       const bool have4 = 8 + half < nchunks;
       if (have4) {
         uint32_t tmp[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_base + (8 + half) * 32, tmp);
+        tmem_ld_32x32b_x32(acc + (8 + half) * 32, tmp);
         tmem_ld_wait();
         pack(tmp, rsv[4], pk4);
       }
       uint32_t raw[4][32];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (2 * i + half < nchunks) tmem_ld_32x32b_x32(tmem_base + lane_base + (2 * i + half) * 32, raw[i]);
+        if (2 * i + half < nchunks) tmem_ld_32x32b_x32(acc + (2 * i + half) * 32, raw[i]);
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(bar_acc_empty & kLeaderMask);
+      if (lane == 0) mbar_arrive_cluster((bar_acc_empty + 8 * buf) & kLeaderMask);
       if (warp == 0) MSC_STAMP(2, tl, 1);
 
       if (!SWIGLU) {
@@ -576,10 +598,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
   }
 }
 
-template <int KIND, int STAGES, bool SWIGLU>
+template <int KIND, bool SWIGLU>
 static int launch_swap(const CUtensorMap* maps, const GemmParams& p, int grid, cudaStream_t stream) {
-  using L = SwapSmem<KIND, STAGES, SWIGLU>;
-  auto kern = gemm_swap_kernel<KIND, STAGES, SWIGLU>;
+  using L = SwapSmem<KIND, SWIGLU>;
+  auto kern = gemm_swap_kernel<KIND, SWIGLU>;
   if (int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kAlloc)) return rc;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t lc = pdl_launch_config(grid, L::kThreads, L::kAlloc, stream, attr);
@@ -613,9 +635,9 @@ int launch_swap_gemm(int kind, const void* a_q, const void* b_q, long long rows_
   if (pairs <= 0) return fail(MSC_ERR_CUDA, "could not query the SM count");
   if (pairs > max_tiles) pairs = (int)max_tiles;
   const int grid = 2 * pairs;
-  if (p.out_q) return launch_swap<KIND_NVFP4, 4, true>(maps, p, grid, stream);
-  if (kind == KIND_NVFP4) return launch_swap<KIND_NVFP4, 4, false>(maps, p, grid, stream);
-  return launch_swap<KIND_MXFP8, 4, false>(maps, p, grid, stream);
+  if (p.out_q) return launch_swap<KIND_NVFP4, true>(maps, p, grid, stream);
+  if (kind == KIND_NVFP4) return launch_swap<KIND_NVFP4, false>(maps, p, grid, stream);
+  return launch_swap<KIND_MXFP8, false>(maps, p, grid, stream);
 }
 
 // ---- w1 with gate and up rows interleaved in blocks of 64 ------------------------------------

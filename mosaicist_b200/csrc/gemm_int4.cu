@@ -67,32 +67,20 @@ struct Int4Smem {
 // should be a sliver.
 template <int TMAX, int GRAIN>
 struct Int4Cursor {
-  int g = 0, base = 0, ttiles = 0, rows = 0, off = 0, width = 0;
-  bool primed = false;
+  int g = 0, rows = 0, off = 0, width = 0;
+  GroupWindow<true> win;
+  static __device__ __forceinline__ int tile_width(int rows) {
+    const int tiles = (rows + TMAX - 1) / TMAX;
+    return tiles ? ((rows + tiles - 1) / tiles + GRAIN - 1) / GRAIN * GRAIN : GRAIN;
+  }
   __device__ __forceinline__ bool seek(const Int4Params& p, int ntiles, int t, int& tt, int& nt) {
-    while (true) {
-      if (!primed) {
-        if (g >= p.l) return false;
-        rows = __shfl_sync(0xffffffffu, __ldg(p.group_rows + g), 0);
-        off = __shfl_sync(0xffffffffu, __ldg(p.group_offsets + g), 0);
-        if (rows < 0) rows = 0;
-        // a group table that reaches beyond the buffers is cut to what the buffers hold
-        if (off < 0 || off >= p.rows_total) rows = 0;
-        else if (rows > p.rows_total - off) rows = p.rows_total - off;
-        ttiles = (rows + TMAX - 1) / TMAX;
-        if (ttiles) {
-          width = ((rows + ttiles - 1) / ttiles + GRAIN - 1) / GRAIN * GRAIN;
-          ttiles = (rows + width - 1) / width;
-        }
-        primed = true;
-      }
-      const int tiles = ttiles * ntiles;
-      if (t < base + tiles) break;
-      base += tiles;
-      ++g;
-      primed = false;
-    }
-    const int u = t - base;
+    int first;
+    if (!win.find(p.l, t,
+                  [&](int gi, int& r, int& o) { load_group(p.group_rows, p.group_offsets, p.rows_total, gi, r, o); },
+                  [=](int r) { const int w = tile_width(r); return (r + w - 1) / w * ntiles; }, g, rows, off, first))
+      return false;
+    width = tile_width(rows);
+    const int u = t - first;
     tt = u / ntiles;
     nt = u - tt * ntiles;
     return true;

@@ -253,6 +253,25 @@ def test_nvfp4_ragged_row_scale_bit_exact(rows_list, n, k, cfg):
     assert np.array_equal(np.where(mask, got, 0), O.bf16_round(want))
 
 
+# the tokens-on-N kernel's ring and accumulators follow from the largest group; groups are found 32 at
+# a time, empty ones among them
+RINGS = [([(i * 7) % 17 * (i % 3 > 0) for i in range(70)], 256, 1152, {"cta_pair": 3, "max_ctas": 6}),
+         ([0] * 33 + [64, 1, 0, 63] + [0] * 30 + [33], 512, 2176, {"cta_pair": 3}),
+         ([65, 128, 0, 96, 17, 127], 256, 1920, {"cta_pair": 3, "max_ctas": 2}),
+         ([129, 160, 0, 1, 145], 512, 1408, {"cta_pair": 3, "max_ctas": 4}),
+         ([161, 160, 12], 256, 1408, {"cta_pair": 3, "max_ctas": 2}),
+         ([0, 0, 0], 256, 256, {"cta_pair": 3})]
+
+
+@pytest.mark.parametrize("rows_list,n,k,cfg", RINGS)
+@pytest.mark.parametrize("kind", ["nvfp4", "mxfp8"])
+def test_tokens_on_n_ring_depths_bit_exact(rows_list, n, k, cfg, kind):
+    if kind == "nvfp4":
+        test_nvfp4_ragged_row_scale_bit_exact(rows_list, n, k, cfg)
+    elif any(rows_list):
+        test_mxfp8_ragged_bit_exact(rows_list, n, k, cfg)
+
+
 def test_random_mxfp8_within_tolerance():
     from mosaicist_b200 import _lib, ops
 

@@ -298,6 +298,12 @@ def test_fused_gemm1_swiglu_quantize_equals_two_kernel_path(rows_list, n, k, swa
     assert np.mean(gq[sl] == O.pack_e2m1(oq)[0]) > 0.99
 
 
+@pytest.mark.parametrize("rows_list,n,k", [([(i * 5) % 17 * (i % 2) for i in range(66)], 128, 640), ([128, 65, 0, 3], 256, 1152),
+                                           ([160, 129, 1], 128, 896)])
+def test_fused_gemm1_ring_depths_equal_two_kernel_path(rows_list, n, k):
+    test_fused_gemm1_swiglu_quantize_equals_two_kernel_path(rows_list, n, k, True)
+
+
 def test_megamoe_layer_replays_from_a_cuda_graph():
     """The whole routed layer is stream-ordered launches without host synchronisation or
     allocation (given `out`), so it captures into one CUDA graph; replays reproduce the eager
