@@ -57,6 +57,8 @@ struct SwapSmem {
 
 // The ring a call runs: groups of up to 64, 128 or any number of tokens.  Weights stream from HBM in a
 // decode step, and what a CTA keeps in flight decides the rate: 7 stages of 24 KB instead of 4 of 44.
+// With the two accumulators of small tiles and the 32-wide group lookup: a routed layer of 16 tokens
+// over 256 experts 510 -> 425 - 452 us, of which the weights alone take 386 at the rate of HBM.
 struct SwapRing {
   int t_bytes;    // tokens of a CTA
   int stage;      // bytes of a stage, a multiple of 1024

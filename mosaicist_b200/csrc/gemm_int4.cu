@@ -24,7 +24,9 @@
 // the converter warps' arrivals; "empty": one commit).  Warps that only wait sleep between probes:
 // their polling took a third of the issue slots from the converters.
 //
-// Measured, 64 groups, n = 2048, k = 7168, cold (the kernel before it, weights expanded into shared
+// Finding a tile's group 32 at a time (GroupWindow) instead of walking the table took the passes of
+// 64 groups, n = 2048, k = 7168 from 177 to 150 - 160 us (1 - 16 rows per group) and from 577 to
+// 538 - 560 us (64 - 512 rows) back to back.  Before that, cold (the kernel before it, weights expanded into shared
 // memory as the N-side operand of 512-row tiles, in brackets): 1 - 16 rows per group 182 us (469),
 // 65 - 128 rows 241 us (472), 64 - 512 rows 417 - 441 us (595), 1320 - 1390 TFLOP/s.  With hundreds
 // of rows the tensor pipe is the limit (it runs into the power cap); with a few rows it is the
