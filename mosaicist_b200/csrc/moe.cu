@@ -25,6 +25,8 @@ template <int PER>
 __global__ void __launch_bounds__(128)
 route_topk_kernel(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ weights,
                   int tokens, int experts, int topk) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= tokens) return;
@@ -99,6 +101,8 @@ __global__ void __launch_bounds__(256)
 moe_plan_kernel(const int* __restrict__ ids, int entries, int expert_first, int experts_local,
                 int* __restrict__ rank, int* __restrict__ group_rows, int* __restrict__ group_offsets,
                 int* __restrict__ total_rows, int* __restrict__ scratch) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   constexpr int kSub = 4;                 // 1024-pair pieces handled between two block barriers
   __shared__ int warp_tot[2][kSub][8];
   __shared__ int is_last;
@@ -232,7 +236,9 @@ constexpr int kMaxTopk = 64;   // pairs of one token the dispatch and combine ke
 // next is quantised.  The quantised bytes depend on the expert only through its global scale,
 // so the row is re-quantised only when that scale differs from the one in shared memory (with
 // one shared input scale a token is quantised once instead of topk times).
-__global__ void __launch_bounds__(128) moe_permute_quantize_kernel(const PermuteParams p, int tokens) {
+__global__ void __launch_bounds__(512) moe_permute_quantize_kernel(const PermuteParams p, int tokens) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   extern __shared__ __align__(16) uint8_t row_smem[];   // 2 x ([hidden/2] values, [hidden/16] scales)
   __shared__ int s_dest[2][kMaxTopk];
   __shared__ float s_gs[2][kMaxTopk];
@@ -298,18 +304,23 @@ __global__ void __launch_bounds__(128) moe_permute_quantize_kernel(const Permute
     }
     if (threadIdx.x == 0) bulk_commit_group();    // one group per token (empty ones count too)
   }
-  if (threadIdx.x == 0) bulk_wait_group_read0();  // the rows are read before the CTA retires
+  if (threadIdx.x == 0) {
+    if (p.sf_rows) bulk_wait_group_read0();   // the rows are read before the CTA retires
+    else bulk_wait_group0();                  // a kernel that starts early follows: they are in place
+  }
 }
 
 // ---- combine -----------------------------------------------------------------------------
-// One CTA per token: the rows holding the token's expert outputs are looked up once, then
-// every thread sums 8 columns at a time over those rows, in the order of the token's pairs,
+// One CTA per token (a few per token when there are not enough of them to fill the chip): the rows
+// holding the token's expert outputs are looked up once, then every thread sums 8 columns at a time over those rows, in the order of the token's pairs,
 // with the loads of up to eight rows issued before the first addition.
 __global__ void __launch_bounds__(256)
 moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ ids,
                      const int* __restrict__ rank, const int* __restrict__ group_offsets,
                      __nv_bfloat16* __restrict__ out, int tokens, int hidden, int topk,
                      int expert_first, int experts_local) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   __shared__ int s_row[kMaxTopk];
   const long long token = blockIdx.x;
   if ((int)threadIdx.x < topk) {
@@ -320,7 +331,7 @@ moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict_
   __syncthreads();
   const int vecs = hidden >> 3;  // 8 bf16 per thread and step
   constexpr int kBatch = 8;
-  for (int vc = threadIdx.x; vc < vecs; vc += blockDim.x) {
+  for (int vc = blockIdx.y * blockDim.x + threadIdx.x; vc < vecs; vc += gridDim.y * blockDim.x) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int k0 = 0; k0 < topk; k0 += kBatch) {
       uint4 raw[kBatch];
@@ -359,9 +370,10 @@ static int launch_plan(const int32_t* ids, int entries, int expert_first, int ex
   if (!ids || !rank || !group_rows || !group_offsets || !total_rows || !scratch)
     return fail(MSC_ERR_BAD_ARG, "NULL pointer");
   if (entries <= 0 || experts_local <= 0) return fail(MSC_ERR_BAD_ARG, "sizes must be positive");
-  moe_plan_kernel<<<experts_local, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      ids, entries, expert_first, experts_local, rank, group_rows, group_offsets, total_rows, scratch);
-  MSC_CUDA_OK(cudaGetLastError());
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t lc = pdl_launch_config(experts_local, 256, 0, static_cast<cudaStream_t>(stream), attr);
+  MSC_CUDA_OK(cudaLaunchKernelEx(&lc, moe_plan_kernel, ids, entries, expert_first, experts_local, rank, group_rows,
+                                 group_offsets, total_rows, scratch));
   return MSC_OK;
 }
 
@@ -431,13 +443,10 @@ int msc_moe_route_topk(const float* logits, int32_t* ids, float* weights, int to
   if (topk < 1 || topk > 32 || topk > experts)
     return msc::fail(MSC_ERR_UNSUPPORTED, "topk=%d must be in [1, 32]", topk);
   const int blocks = (tokens + 3) / 4;
-  if (experts <= 256)
-    msc::route_topk_kernel<8><<<blocks, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        logits, ids, weights, tokens, experts, topk);
-  else
-    msc::route_topk_kernel<msc::kMaxExpertsPerLane><<<blocks, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        logits, ids, weights, tokens, experts, topk);
-  MSC_CUDA_OK(cudaGetLastError());
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t lc = msc::pdl_launch_config(blocks, 128, 0, static_cast<cudaStream_t>(stream), attr);
+  auto kern = experts <= 256 ? msc::route_topk_kernel<8> : msc::route_topk_kernel<msc::kMaxExpertsPerLane>;
+  MSC_CUDA_OK(cudaLaunchKernelEx(&lc, kern, logits, ids, weights, tokens, experts, topk));
   return MSC_OK;
 }
 
@@ -464,15 +473,19 @@ int msc_moe_permute_quantize(const void* tokens_bf16, const int32_t* ids, const 
   p.ids = ids; p.weights = weights; p.rank = rank; p.group_offsets = group_offsets; p.gs = input_gs;
   p.q = static_cast<uint8_t*>(a_q); p.sf = static_cast<uint8_t*>(a_sf);
   p.row_weight = row_weight; p.row_token = row_token;
-  // the staged form needs scale rows that bulk copies can carry (a multiple of 16 bytes)
-  const bool staged = sf_rows != nullptr;
-  if (staged) {
+  // the staged form needs scale rows that bulk copies can carry (a multiple of 16 bytes).  Up to 4096
+  // rows its second launch costs more than the 4-byte stores it saves, and the tiling is written
+  // directly.  With every launch here set up under the kernel before it, the routed layer takes, us:
+  // 16 tokens, 64 experts, top-4, 2048 x 512 63.4 -> 50.4; 512 tokens, 2048 x 768 87.0 -> 73.9; 90
+  // tokens, 128 experts, top-8, 2688 x 640 128.0 -> 118.3; 1 token, 256 experts, 7168 x 2048 88.4 -> 69.6.
+  const bool staged = sf_rows != nullptr && (long long)tokens * topk > 4096;
+  if (sf_rows) {
     if (hidden % 256) return msc::fail(MSC_ERR_BAD_ARG, "sf_rows needs hidden %% 256 == 0, got %d", hidden);
     if (rows_cap <= 0 || rows_cap % 128) return msc::fail(MSC_ERR_BAD_ARG, "rows_cap=%d must be a positive multiple of 128", rows_cap);
     if (reinterpret_cast<uintptr_t>(sf_rows) % 16 || reinterpret_cast<uintptr_t>(a_sf) % 16)
       return msc::fail(MSC_ERR_BAD_ARG, "sf_rows and a_sf must be 16-byte aligned");
   }
-  p.sf_rows = static_cast<uint8_t*>(sf_rows);
+  p.sf_rows = staged ? static_cast<uint8_t*>(sf_rows) : nullptr;
   p.entries = tokens * topk; p.hidden = hidden; p.topk = topk;
   p.expert_first = expert_first; p.experts_local = experts_local;
   if (topk > msc::kMaxTopk) return msc::fail(MSC_ERR_UNSUPPORTED, "topk=%d exceeds %d", topk, msc::kMaxTopk);
@@ -483,12 +496,15 @@ int msc_moe_permute_quantize(const void* tokens_bf16, const int32_t* ids, const 
   if (smem > 48 * 1024)
     if (int rc = msc::allow_dynamic_smem(reinterpret_cast<const void*>(msc::moe_permute_quantize_kernel), 200 * 1024))
       return rc;
-  // enough CTAs to fill every SM (16 x 128 threads), each walking its share of the tokens
+  // enough CTAs to fill every SM (16 x 128 threads), each walking its share of the tokens; wide CTAs
+  // for a few tokens, whose rows are then one step long
   const int sms = msc::num_sms();
   if (sms <= 0) return msc::fail(MSC_ERR_CUDA, "could not query the SM count");
   const int grid = tokens < 16 * sms ? tokens : 16 * sms;
-  msc::moe_permute_quantize_kernel<<<grid, 128, smem, static_cast<cudaStream_t>(stream)>>>(p, tokens);
-  MSC_CUDA_OK(cudaGetLastError());
+  const int threads = tokens <= 2 * sms ? 512 : 128;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t lc = msc::pdl_launch_config(grid, threads, smem, static_cast<cudaStream_t>(stream), attr);
+  MSC_CUDA_OK(cudaLaunchKernelEx(&lc, msc::moe_permute_quantize_kernel, p, tokens));
   if (staged)
     return msc::launch_sf_swizzle(sf_rows, a_sf, 1, rows_cap, hidden / 64, total_rows,
                                   static_cast<cudaStream_t>(stream));
@@ -502,10 +518,15 @@ int msc_moe_unpermute(const void* y, const int32_t* ids, const int32_t* rank,
   if (tokens <= 0 || topk <= 0 || experts_local <= 0) return msc::fail(MSC_ERR_BAD_ARG, "sizes must be positive");
   if (hidden <= 0 || hidden % 8) return msc::fail(MSC_ERR_BAD_ARG, "hidden=%d must be a multiple of 8", hidden);
   if (topk > msc::kMaxTopk) return msc::fail(MSC_ERR_UNSUPPORTED, "topk=%d exceeds %d", topk, msc::kMaxTopk);
-  msc::moe_unpermute_kernel<<<(unsigned)tokens, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(y), ids, rank, group_offsets,
-      static_cast<__nv_bfloat16*>(out), tokens, hidden, topk, expert_first, experts_local);
-  MSC_CUDA_OK(cudaGetLastError());
+  const int sms = msc::num_sms();
+  if (sms <= 0) return msc::fail(MSC_ERR_CUDA, "could not query the SM count");
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t lc = msc::pdl_launch_config(tokens, 256, 0, static_cast<cudaStream_t>(stream), attr);
+  if (tokens < 2 * sms) lc.gridDim.y = (unsigned)((hidden / 8 + 255) / 256);
+  else lc.numAttrs = 0;   // thousands of CTAs waiting beside the GEMM before it would only be in its way
+  MSC_CUDA_OK(cudaLaunchKernelEx(&lc, msc::moe_unpermute_kernel, static_cast<const __nv_bfloat16*>(y), ids, rank,
+                                 group_offsets, static_cast<__nv_bfloat16*>(out), tokens, hidden, topk, expert_first,
+                                 experts_local));
   return MSC_OK;
 }
 

@@ -338,3 +338,40 @@ def test_megamoe_layer_replays_from_a_cuda_graph():
         eager = layer.forward(tokens, logits)
         assert torch.equal(replayed, eager) and int((eager != 0).sum()) > eager.numel() // 2
     assert _lib.status_word() == 0
+
+
+@pytest.mark.parametrize("tokens_n", [1, 296, 297, 512, 520])   # wide and narrow CTAs; direct and staged scales (4096 rows)
+def test_dispatch_and_combine_forms_agree(tokens_n):
+    """Scales written directly and through the staging buffer are the same bytes in live rows, and a
+    token's combined row does not depend on how many tokens (CTAs per token) the call has."""
+    from mosaicist_b200 import _lib
+    from mosaicist_b200.formats import from_mma_scale_layout
+    from mosaicist_b200.moe import MegaMoE, _host_ops
+
+    E, k, h, n = 32, 8, 4352, 128
+    rng = torch.Generator(device="cuda").manual_seed(tokens_n)
+    u8 = lambda *s: torch.randint(0, 256, s, dtype=torch.uint8, device="cuda", generator=rng)
+    one = torch.ones((E,), device="cuda")
+    sf1 = torch.full((E, 2 * n // 128, h // 64, 32, 16), 0x38, dtype=torch.uint8, device="cuda")     # e4m3 1.0
+    sf2 = torch.full((E, h // 128, n // 64, 32, 16), 0x38, dtype=torch.uint8, device="cuda")
+    layer = MegaMoE(u8(E, 2 * n, h // 2), sf1, one, one * 1e-3, u8(E, h, n // 2), sf2, one, one, one * 500, one * 50,
+                    topk=k, max_tokens=tokens_n)
+    x = torch.randn((tokens_n, h), device="cuda", generator=rng).bfloat16()
+    logits = torch.randn((tokens_n, E), device="cuda", generator=rng)
+    out = layer.forward(x, logits)
+    want_q, want_sf = layer.a_q.clone(), layer.a_sf.clone()
+    layer.a_q.fill_(0), layer.a_sf.fill_(0)
+    assert layer.sf_rows is not None
+    layer.sf_rows = None
+    _host_ops.moe_dispatch(layer, x, None)
+    live = torch.zeros((layer.rows_cap,), dtype=torch.bool)
+    for o, r in zip(layer.group_offsets.tolist(), layer.group_rows.tolist()):
+        live[o:o + r] = True
+    assert int(live.sum()) == tokens_n * k
+    assert torch.equal(layer.a_q.cpu()[live], want_q.cpu()[live])
+    sf = [torch.from_numpy(from_mma_scale_layout(s.cpu().numpy(), layer.rows_cap).copy()) for s in (layer.a_sf, want_sf)]
+    assert torch.equal(sf[0][live], sf[1][live])
+    few = min(tokens_n, 16)
+    assert torch.equal(_host_ops.moe_combine(layer, x[:few], None), out[:few])
+    assert int((out != 0).sum()) > out.numel() // 2
+    assert _lib.status_word() == 0
