@@ -69,9 +69,8 @@ const char* msc_last_error(void);
  * Call it when no launch is being issued; later calls encode their maps again. */
 int msc_shutdown(void);
 
-/* Path of the PTX text of this library's kernels (written next to the .so at build time),
- * so a capture module can drop it where the reference's collect_artifacts looks
- * (src/mosaicist/capture.py:81-116).  Host string, owned by the library. */
+/* An empty string: PTX text of the kernels is not built (the symbol stays for callers that link
+ * against it).  A capture module leaves the kernel's CUDA source and the ptxas log instead. */
 const char* msc_ptx_path(void);
 
 /* Reads and clears the device status word of the current device (0 = no kernel gave up).

@@ -1,4 +1,4 @@
-"""Builds libmosaicist_sm100a.so (and the PTX text beside it) in-tree with nvcc.
+"""Builds libmosaicist_sm100a.so in-tree with nvcc.
 
     python -m mosaicist_b200.build [--force] [--debug]
 
@@ -20,13 +20,6 @@ import sys
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libmosaicist_sm100a.so"
-PTX = PKG / "libmosaicist_sm100a.ptx"
-#: PTX text per GEMM translation unit; the first is the default kernel and sits where
-#: msc_ptx_path() points, the others beside it with a suffix
-PTX_UNITS = {"pair": ("gemm_blockscaled_pair.cu", PTX),
-             "single": ("gemm_blockscaled.cu", PKG / "libmosaicist_sm100a.single.ptx"),
-             "dense": ("gemm_dense_f16.cu", PKG / "libmosaicist_sm100a.dense.ptx"),
-             "int4": ("gemm_int4.cu", PKG / "libmosaicist_sm100a.int4.ptx")}
 PTXAS_LOG = PKG / "libmosaicist_sm100a.ptxas.log"
 DEBUG_LIB = PKG / "libmosaicist_sm100a_debug.so"
 
@@ -39,7 +32,7 @@ def sources() -> list[pathlib.Path]:
 
 
 def _stale() -> bool:
-    if not LIB.exists() or not all(dst.exists() for _, dst in PTX_UNITS.values()):
+    if not LIB.exists():
         return True
     built = LIB.stat().st_mtime
     deps = list(CSRC.glob("*")) + [PKG.parent / "include" / "mosaicist_sm100a.h"]
@@ -66,12 +59,6 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         raise RuntimeError("nvcc failed:\n" + res.stderr[-4000:])
     if verbose:
         print(res.stderr)
-    # PTX text of the GEMM kernels: what a capture module hands to the PTX fingerprinter
-    for src, dst in PTX_UNITS.values():
-        cmd = [nvcc, *ARCH, *COMMON, "-ptx", "-o", str(dst), str(CSRC / src)]
-        res = subprocess.run(cmd, capture_output=True, text=True)
-        if res.returncode != 0:
-            raise RuntimeError("nvcc -ptx failed:\n" + res.stderr[-4000:])
     return LIB
 
 

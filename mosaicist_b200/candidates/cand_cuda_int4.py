@@ -65,10 +65,7 @@ def build():
     k = from_env(DEFAULTS)
     a, b_q, scales, offs, rows = _inputs()
     out = torch.zeros((a.shape[0], N), dtype=torch.bfloat16, device=a.device)
-    if int(k["fused"]):
-        drop_artifacts("int4", "gemm_int4_pair_kernelILi256E")
-    else:
-        drop_artifacts("dense", "gemm_dense_f16_kernelILi6ELb1ELb0E")
+    drop_artifacts("gemm_int4.cu" if int(k["fused"]) else "gemm_dense_f16.cu")
 
     def fn():
         return ops.mixed_grouped_gemm_int4(a, b_q, scales, offs, rows, None, GROUP_SIZE, out=out,

@@ -7,7 +7,6 @@
 #include <atomic>
 #include <memory>
 #include <mutex>
-#include <string>
 #include <set>
 #include <unordered_map>
 #include <utility>
@@ -213,19 +212,7 @@ int msc_shutdown(void) {
 
 const char* msc_last_error(void) { return msc::g_err; }
 
-const char* msc_ptx_path(void) {
-  static std::string path;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    Dl_info info;
-    if (dladdr(reinterpret_cast<void*>(&msc_version), &info) && info.dli_fname) {
-      std::string so(info.dli_fname);
-      size_t dot = so.rfind(".so");
-      path = (dot == std::string::npos ? so : so.substr(0, dot)) + ".ptx";
-    }
-  });
-  return path.c_str();
-}
+const char* msc_ptx_path(void) { return ""; }
 
 int msc_status_word_read(int* out) {
   if (!out) return msc::fail(MSC_ERR_BAD_ARG, "out is NULL");

@@ -39,8 +39,6 @@ def test_library_exports_every_declared_symbol(lib):
         assert name in _lib.SIGNATURES, f"{name} has no ctypes signature"
     assert sorted(_lib.SIGNATURES) == names
     assert lib.msc_version() >= 1
-    assert lib.msc_ptx_path().decode().endswith("libmosaicist_sm100a.ptx")
-    assert pathlib.Path(lib.msc_ptx_path().decode()).exists()
 
 
 def test_bad_arguments_are_rejected_with_a_message(lib):
@@ -260,25 +258,22 @@ def test_torch_custom_op_is_registered_and_shape_propagates():
         assert tuple(y.shape) == (2, 256, 512) and y.dtype == torch.bfloat16
 
 
-def test_dropped_ptx_is_reduced_to_the_running_instantiation(lib, tmp_path, monkeypatch):
-    """The capture module leaves a PTX holding only the kernel instantiation that runs (the
-    fingerprinter picks the entry with the most instructions)."""
-    import re
+@pytest.mark.parametrize("module", ["gemm", "moe", "mxfp8", "dense", "int4"])
+def test_capture_modules_leave_sources_and_the_ptxas_log(lib, module, tmp_path, monkeypatch):
+    """Compiler output of the kernels is neither built beside the library nor left in a bundle: a
+    capture module leaves the CUDA sources of the kernels that can run and the ptxas log."""
+    import inspect
 
+    from mosaicist_b200 import _lib
     from mosaicist_b200.candidates import _common
 
-    toy = (".version 8.8\n.target sm_100a\n.extern .shared .b8 s[];\n"
-           ".visible .entry kA_ILi1E(\n .param .u64 p\n)\n{\n { nested } \n ret;\n}\n"
-           ".visible .entry kB_ILi2E(\n .param .u64 p\n)\n.maxntid 320\n{\n ret;\n}\n")
-    red = _common.only_entry(toy, "kB_ILi2E")
-    assert "kB_ILi2E" in red and "kA_ILi1E" not in red and red.startswith(".version 8.8") and ".maxntid 320" in red
-    assert _common.only_entry(toy, "missing") == toy
+    assert lib.msc_ptx_path() == b"" and not list(_lib.PKG.glob("*.ptx"))
+    text = inspect.getsource(__import__(f"mosaicist_b200.candidates.cand_cuda_{module}", fromlist=["build"]))
+    names = sorted(set(re.findall(r'"(gemm_\w+\.cu)"', text)))
+    assert names and all((_lib.PKG / "csrc" / n).exists() for n in names)
     monkeypatch.setenv("MOSAIC_GPU_DUMP_TO", str(tmp_path))
-    _common.drop_artifacts("pair", "gemm_pair_kernelILi0ELi5ELb0ELb0ELb0E")
-    text = next(tmp_path.glob("*.ptx")).read_text()
-    entries = re.findall(r"^\.visible \.entry (\S+)\(", text, re.M)
-    assert len(entries) == 1 and "gemm_pair_kernelILi0ELi5ELb0ELb0ELb0E" in entries[0]
-    assert list(tmp_path.glob("ptxas*"))
+    _common.drop_artifacts(*names)
+    assert sorted(f.name for f in tmp_path.iterdir()) == sorted(names + ["ptxas_mosaicist_sm100a.log"])
 
 
 def test_bench_reference_arm_runs_on_the_cpu_and_prints_the_contract_line():
@@ -296,34 +291,3 @@ def test_bench_reference_arm_runs_on_the_cpu_and_prints_the_contract_line():
     assert line["cpu_baseline"]["kind"] == "port" and line["cpu_baseline"]["cores"] >= 1
     assert line["cpu_baseline"]["value"] == line["value"] > 0
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["e2e"]["d2h_bytes_per_step"] == 0
-
-
-@pytest.mark.parametrize("kernel,entry", [("pair", "gemm_pair_kernelILi0ELi5ELb0ELb0ELb0E"),
-                                          ("single", "gemm_blockscaled_kernelILi0ELi128ELi5E"),
-                                          ("dense", "gemm_dense_f16_kernelILi6ELb0ELb0E")])
-def test_reference_fingerprinter_accepts_the_dropped_ptx(kernel, entry, tmp_path, monkeypatch, lib):
-    """What a capture module leaves in the dump directory goes through the reference's own PTX
-    parser and fingerprinter (src/mosaicist/ptx/parse.py, features.py:151): it parses, its largest
-    entry is the instantiation that was asked for, and the fingerprint sees tensor-core and TMA
-    instructions."""
-    from oracle.stage_reference import staged_path
-
-    ref = staged_path()
-    if ref is None:
-        pytest.skip("the reference's package is neither staged (oracle/stage_reference.py) nor in MOSAICIST_REFERENCE")
-    monkeypatch.syspath_prepend(str(ref))
-    monkeypatch.setenv("MOSAIC_GPU_DUMP_TO", str(tmp_path))
-    from mosaicist.ptx.features import fingerprint
-    from mosaicist.ptx.parse import parse
-    from mosaicist_b200.candidates._common import drop_artifacts
-
-    drop_artifacts(kernel, entry)
-    files = list(tmp_path.glob("*.ptx"))
-    assert len(files) == 1
-    text = files[0].read_text()
-    mod = parse(text)
-    assert entry in mod.entry(None).name and mod.target == "sm_100a"
-    fp = fingerprint(text, ptxas_log=(tmp_path / "ptxas_mosaicist_sm100a.log").read_text())
-    ops = " ".join(i.opcode for i in mod.entry(None).instrs)
-    assert "tcgen05.mma" in ops and "cp.async.bulk.tensor" in ops
-    assert fp is not None

@@ -1,11 +1,10 @@
 """The capture modules driven by the reference's OWN capture stage on a GPU.
 
 `mosaicist.capture.capture()` (src/mosaicist/capture.py:229-271) imports a module, calls its
-build(), runs the callable under CUPTI activity tracing, gathers the PTX / ptxas log the module
+build(), runs the callable under CUPTI activity tracing, gathers the ptxas log the module
 dropped, saves out0.npy and - from the module's reference() - oracle0.npy, and writes a bundle.
 These tests run exactly that, unchanged, on this library's modules and check what the
-convergence loop would read next: the PTX fingerprints and its largest entry is the kernel that
-ran, the numerics gate passes on the saved arrays, the launch record is the kernel's, and the
+convergence loop would read next: the numerics gate passes on the saved arrays, the launch record is the kernel's, and the
 CUPTI per-launch time agrees with CUDA-event timing.
 
 Needs the reference's Python package (staged by oracle/stage_reference.py, or $MOSAICIST_REFERENCE)
@@ -71,20 +70,15 @@ def _event_us(fn, args, reps=30):
 def test_reference_capture_stage_drives_the_module(reference_capture, name, measure, kernel):
     C, out = reference_capture
     from mosaicist.bundle import Bundle
-    from mosaicist.ptx.parse import parse
     from mosaicist.verify.numerics import compare_outputs
     from mosaicist.verify.formats import round_to_format
 
     entry = f"mosaicist_b200.candidates.{name}"
     bundle = C.capture(entry, "pallas", out, reps=30, warmup=5, arch="sm_100a", measure=measure)
 
-    # artifacts: a PTX whose largest entry is the kernel that ran, the ptxas log, a bundle that loads
-    ptx = (out / "kernel.ptx").read_text()
-    assert kernel in parse(ptx).entry(None).name
-    assert (out / "ptxas.log").exists()
-    loaded = Bundle.load(out)
-    fp = loaded.fingerprint()
-    assert fp is not None and loaded.kind == "candidate" and loaded.ptx == "kernel.ptx"
+    # artifacts: the ptxas log, a bundle that loads
+    assert kernel in (out / "ptxas.log").read_text()
+    assert Bundle.load(out).kind == "candidate"
 
     # launch record of the dominant kernel: a persistent grid of CTA pairs, 320 threads
     assert bundle.launch.block == [320, 1, 1] and bundle.launch.cluster == [2, 1, 1]
