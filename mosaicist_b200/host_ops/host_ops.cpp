@@ -18,6 +18,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
@@ -828,6 +829,14 @@ TORCH_LIBRARY_IMPL(mosaicist_sm100a, CUDA, m) {
   m.impl("gemm_f16", op_gemm_f16);
   m.impl("grouped_gemm_bf16_int4_ragged", op_grouped_gemm_bf16_int4_ragged);
   m.impl("moe_masked", op_moe_masked);
+}
+// No operator has a derivative: a backward pass through one raises.  (Without a kernel under this
+// key torch only warns and leaves the operator's share out of the gradients.)
+TORCH_LIBRARY_IMPL(mosaicist_sm100a, Autograd, m) {
+  for (const char* name : {"grouped_gemm_nvfp4", "grouped_gemm_nvfp4_ragged", "quantize_nvfp4", "silu_mul_quantize_nvfp4",
+                           "global_scale_for", "quantize_mxfp8", "grouped_gemm_mxfp8_ragged", "gemm_f16",
+                           "grouped_gemm_bf16_int4_ragged", "moe_masked"})
+    m.impl(name, torch::autograd::autogradNotImplementedFallback());
 }
 
 }  // namespace
