@@ -321,6 +321,13 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (!cur.seek(p, ntiles, t, mt, nt)) break;
       const int buf = tl % kAccBufs;
       const uint32_t aph = (tl / kAccBufs) & 1;
+      // the factors arrive while the main loop runs
+      const int row_warp = mt * 128 + quad * 32;
+      const bool valid = row_warp + lane < cur.rows;
+      const bool whole_warp = row_warp + 32 <= cur.rows;
+      const size_t out_row = (size_t)cur.off + row_warp + lane;
+      float scale = group_alpha(p, cur.g);
+      if (p.row_scale && valid) scale *= ld_ordered(p.row_scale + out_row);
       // one lane per warp waits; the others park on the warp vote instead of polling
       bool ok = true;
       if (lane == 0) ok = mbar_wait_bounded(bar_acc_full + 8 * buf, aph, abort_flag, p.status, 4);
@@ -328,12 +335,6 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (!ok) break;
       tc_fence_after_sync();
       if (warp == 0) MSC_STAMP(2, tl, 0);
-      const int row_warp = mt * 128 + quad * 32;
-      const bool valid = row_warp + lane < cur.rows;
-      const bool whole_warp = row_warp + 32 <= cur.rows;
-      const size_t out_row = (size_t)cur.off + row_warp + lane;
-      float scale = group_alpha(p, cur.g);
-      if (p.row_scale && valid) scale *= __ldg(p.row_scale + out_row);
 
       uint32_t v[4][32];
 #pragma unroll

@@ -358,18 +358,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int t = pair;; t += npairs, ++tl) {
       int mt, nt;
       if (!cur.seek(p, ntiles, t, mt, nt)) break;
+      // the factors arrive while the main loop runs
+      const int row_warp = (2 * mt + (int)rank) * 128 + quad * 32;
+      const bool valid = row_warp + lane < cur.rows;
+      const bool whole_warp = row_warp + 32 <= cur.rows;
+      const size_t out_row = (size_t)cur.off + row_warp + lane;
+      float scale = group_alpha(p, cur.g);
+      if (p.row_scale && valid) scale *= ld_ordered(p.row_scale + out_row);
+      const float gs = SWIGLU && valid ? ld_ordered(p.out_gs + cur.g) : 0.0f;
       bool ok = true;
       if (lane == 0) ok = mbar_wait_bounded(bar_acc_full, tl & 1, abort_flag, p.status, 4);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
       if (warp == 0) MSC_STAMP(2, tl, 0);
-      const int row_warp = (2 * mt + (int)rank) * 128 + quad * 32;
-      const bool valid = row_warp + lane < cur.rows;
-      const bool whole_warp = row_warp + 32 <= cur.rows;
-      const size_t out_row = (size_t)cur.off + row_warp + lane;
-      float scale = group_alpha(p, cur.g);
-      if (p.row_scale && valid) scale *= __ldg(p.row_scale + out_row);
 
       uint32_t v[4][32];
       if (SWIGLU) {
@@ -398,7 +400,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         // thread quantises its four 16-column blocks: 32 bytes of e2m1 and one scale word,
         // which is one unit of the tiled scale layout the second GEMM reads.
         if (valid) {
-          const float gs = __ldg(p.out_gs + cur.g);
           const int width = p.n >> 1;                       // columns of the activation
           const int col = nt * 128 + slab * 64;             // first output column of this thread
           uint32_t q8[8], sfw = 0;
@@ -432,7 +433,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         // Every row goes to its own destination (another GPU's memory included): the lane
         // stages its row's 128 bf16 columns linearly and sends them as one 256-byte bulk copy.
         // A lane only ever touches its own staging row, so no warp-level ordering is needed.
-        const int dcode = valid ? __ldg(p.row_dest + out_row) : -1;
+        const int dcode = valid ? ld_ordered(p.row_dest + out_row) : -1;
         bulk_wait_group_read0();   // this lane's previous copy has left its staging row
         const uint32_t rowaddr = box0 + lane * L::kScatterPitch;
 #pragma unroll

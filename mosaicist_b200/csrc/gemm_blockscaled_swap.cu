@@ -191,7 +191,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
   // the largest group decides the depth of the ring and whether two accumulators fit; every role of
   // both CTAs reads the same table
   int most = 0;
-  for (int g = lane; g < p.l; g += 32) most = max(most, __ldg(p.group_rows + g));
+  for (int g = lane; g < p.l; g += 32) most = max(most, ld_ordered(p.group_rows + g));
   most = __reduce_max_sync(0xffffffffu, most);
   const SwapRing ring = SwapRing::make<L>(most);
   const bool two_acc = most <= kAccCol;
@@ -363,8 +363,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
         const int tok = (2 * i + half) * 32 + lane;
-        rsv[i] = (!SWIGLU && p.row_scale && tok < tn) ? __ldg(p.row_scale + (size_t)cur.off + (size_t)tt * 256 + tok) : 1.0f;
+        rsv[i] = (!SWIGLU && p.row_scale && tok < tn) ? ld_ordered(p.row_scale + (size_t)cur.off + (size_t)tt * 256 + tok) : 1.0f;
       }
+      const float alpha = group_alpha(p, cur.g);
+      const float gs = SWIGLU ? ld_ordered(p.out_gs + cur.g) : 0.0f;
       bool ok = true;
       const int buf = two_acc ? (tl & 1) : 0;
       const uint32_t use = two_acc ? (uint32_t)(tl >> 1) : (uint32_t)tl;
@@ -388,7 +390,6 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
       if (!ok) break;
       tc_fence_after_sync();
       if (warp == 0) MSC_STAMP(2, tl, 0);
-      const float alpha = group_alpha(p, cur.g);
       const size_t row0 = (size_t)cur.off + (size_t)tt * 256;   // first token row of the tile
       // 32 tokens of this lane's row, as read from TMEM -> alpha (and the tokens' row scales)
       // applied, rounded to bf16, two tokens per register
@@ -506,7 +507,6 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w,
       // rounded to bf16 (gemm1_silu_quantize.py:195-197), into a shared [token][row] tile; after
       // a barrier thread (token, 16-column block) activates (nvfp4.py:81-88) and quantises its
       // block.
-      const float gs = __ldg(p.out_gs + cur.g);
       const int width = p.n >> 1;                       // columns of the activation
       const int col0 = (nt * 2 + (int)rank) * 64;       // first activation column of this CTA
       const uint32_t cbase = sbase + L::kOffC;

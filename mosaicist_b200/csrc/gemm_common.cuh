@@ -67,9 +67,9 @@ extern int g_debug_flags;
 // Factor of a group's accumulators.
 __device__ __forceinline__ float group_alpha(const GemmParams& p, int g) {
   if (!p.alpha) return 1.0f;
-  const float a = __ldg(p.alpha + g);
+  const float a = ld_ordered(p.alpha + g);
   if (!p.alpha_gs_a) return a;
-  return __fdiv_rn(a, __fmul_rn(__ldg(p.alpha_gs_a + g), __ldg(p.alpha_gs_b + g)));
+  return __fdiv_rn(a, __fmul_rn(ld_ordered(p.alpha_gs_a + g), ld_ordered(p.alpha_gs_b + g)));
 }
 
 // Finds the group of a tile, 32 groups at a time: lane i of the (converged) warp holds the running
@@ -122,8 +122,8 @@ struct GroupWindow {
 // expert-parallel step, a stale table after a timed-out wait) is cut to what the buffers hold.
 __device__ __forceinline__ void load_group(const int* group_rows, const int* group_offsets, int rows_total, int g,
                                            int& rows, int& off) {
-  rows = max(__ldg(group_rows + g), 0);
-  off = __ldg(group_offsets + g);
+  rows = max(ld_ordered(group_rows + g), 0);
+  off = ld_ordered(group_offsets + g);
   if (off < 0 || off >= rows_total) rows = 0;
   else if (rows > rows_total - off) rows = rows_total - off;
 }
@@ -138,10 +138,10 @@ struct TileCursor {
       if (!primed) {
         if (g >= p.l) return false;
         // every lane reads the same word; the broadcast tells the compiler so
-        rows = p.group_rows ? __shfl_sync(0xffffffffu, __ldg(p.group_rows + g), 0) : p.m_stride;
+        rows = p.group_rows ? __shfl_sync(0xffffffffu, ld_ordered(p.group_rows + g), 0) : p.m_stride;
         if (rows < 0) rows = 0;
         if (p.m_stride > 0 && rows > p.m_stride) rows = p.m_stride;
-        off = p.group_offsets ? __shfl_sync(0xffffffffu, __ldg(p.group_offsets + g), 0)
+        off = p.group_offsets ? __shfl_sync(0xffffffffu, ld_ordered(p.group_offsets + g), 0)
                               : g * p.m_stride;
         // a group table that reaches beyond the buffers (an overflowing expert-parallel step,
         // a stale table after a timed-out wait) is cut to what the buffers hold

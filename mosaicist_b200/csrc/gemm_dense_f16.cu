@@ -252,6 +252,7 @@ gemm_dense_f16_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (t >= total_tiles) break;
         dense_tile(p, t, mt, nt);
       }
+      const float scale = (GROUPED && p.g.alpha) ? ld_ordered(p.g.alpha + cur.g) : 1.0f;   // during the main loop
       const int buf = kOneAcc ? 0 : (tl & 1);
       const uint32_t use = kOneAcc ? (uint32_t)tl : (uint32_t)(tl >> 1);
       bool ok = true;
@@ -265,7 +266,6 @@ gemm_dense_f16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int row0 = (GROUPED ? cur.off : 0) + row_in;
       // wide tiles: slab w / 4 drains one whole 256-column accumulator, 128 columns per pass
       const int colb = WIDE ? (nt * 512 + slab * 256) * 2 : (nt * 256 + slab * 128) * 2;   // byte column
-      const float scale = (GROUPED && p.g.alpha) ? __ldg(p.g.alpha + cur.g) : 1.0f;
       const bool ragged = GROUPED && row_in + 32 > cur.rows;
       // The warp's 128 columns are drained in one pass (two for its 256 columns of a wide tile); the
       // accumulator is handed back after the last read.

@@ -345,7 +345,7 @@ __device__ __forceinline__ void gemm_int4_body(const CUtensorMap& tmap_w, const 
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           if (i == 1 && shared_scale) break;
-          if (grp[i] < groups_k) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v[i]) : "l"(srow + grp[i]));
+          if (grp[i] < groups_k) asm volatile("ld.global.u16 %0, [%1];" : "=h"(v[i]) : "l"(srow + grp[i]));
           grp[i] += step_groups;
           if (!whole_steps) {
             rem[i] += step_rem;
@@ -421,9 +421,9 @@ __device__ __forceinline__ void gemm_int4_body(const CUtensorMap& tmap_w, const 
       const int tn = cur.tokens(tt);
       const int buf = kTwoAcc ? (tl & 1) : 0;
       const uint32_t use = kTwoAcc ? (uint32_t)(tl >> 1) : (uint32_t)tl;
+      const float alpha = p.alpha ? ld_ordered(p.alpha + cur.g) : 1.0f;   // arrives during the main loop
       if (!warp_wait_relaxed(bar_acc_full + 8 * buf, use & 1u, abort_flag, p.status, 7, 400)) break;
       tc_fence_after_sync();
-      const float alpha = p.alpha ? __ldg(p.alpha + cur.g) : 1.0f;
       const int nchunks = (tn + 31) >> 5;
       // the accumulator goes back before anything is stored: 32 tokens of this lane's column at a
       // time, scaled and rounded, two tokens per register

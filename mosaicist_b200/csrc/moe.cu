@@ -23,7 +23,7 @@ constexpr int kMaxExpertsPerLane = 32;  // experts <= 1024
 // PER: register slots per lane (experts / 32 rounded up to 8 or 32); unused slots hold -inf / -1.
 template <int PER>
 __global__ void __launch_bounds__(128)
-route_topk_kernel(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ weights,
+route_topk_kernel(const float* logits, int* __restrict__ ids, float* __restrict__ weights,
                   int tokens, int experts, int topk) {
   grid_dependency_wait();
   grid_launch_dependents();
@@ -36,7 +36,7 @@ route_topk_kernel(const float* __restrict__ logits, int* __restrict__ ids, float
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    v[i] = (i < per) ? __ldg(row + lane + 32 * i) : -INFINITY;
+    v[i] = (i < per) ? ld_ordered(row + lane + 32 * i) : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
 #pragma unroll
@@ -98,7 +98,7 @@ route_topk_kernel(const float* __restrict__ logits, int* __restrict__ ids, float
 // group's row count.  The last block to finish (a ticket counter in `scratch`) turns the
 // counts into 128-aligned group offsets and resets the ticket for the next call.
 __global__ void __launch_bounds__(256)
-moe_plan_kernel(const int* __restrict__ ids, int entries, int expert_first, int experts_local,
+moe_plan_kernel(const int* ids, int entries, int expert_first, int experts_local,
                 int* __restrict__ rank, int* __restrict__ group_rows, int* __restrict__ group_offsets,
                 int* __restrict__ total_rows, int* __restrict__ scratch) {
   grid_dependency_wait();
@@ -123,12 +123,12 @@ moe_plan_kernel(const int* __restrict__ ids, int entries, int expert_first, int 
       const int i0 = base + j * 1024 + threadIdx.x * 4;
       v[j] = make_int4(-1, -1, -1, -1);
       if (vec && i0 + 3 < entries) {
-        v[j] = __ldg(reinterpret_cast<const int4*>(ids + i0));
+        v[j] = ld_ordered(reinterpret_cast<const int4*>(ids + i0));
       } else {
-        if (i0 < entries) v[j].x = __ldg(ids + i0);
-        if (i0 + 1 < entries) v[j].y = __ldg(ids + i0 + 1);
-        if (i0 + 2 < entries) v[j].z = __ldg(ids + i0 + 2);
-        if (i0 + 3 < entries) v[j].w = __ldg(ids + i0 + 3);
+        if (i0 < entries) v[j].x = ld_ordered(ids + i0);
+        if (i0 + 1 < entries) v[j].y = ld_ordered(ids + i0 + 1);
+        if (i0 + 2 < entries) v[j].z = ld_ordered(ids + i0 + 2);
+        if (i0 + 3 < entries) v[j].w = ld_ordered(ids + i0 + 3);
       }
     }
     unsigned b[kSub][4];
@@ -254,13 +254,13 @@ __global__ void __launch_bounds__(512) moe_permute_quantize_kernel(const Permute
     if (threadIdx.x == 0) bulk_wait_group_read1();
     if ((int)threadIdx.x < p.topk) {
       const int k = threadIdx.x;
-      const int e = __ldg(p.ids + token * p.topk + k) - p.expert_first;
+      const int e = ld_ordered(p.ids + token * p.topk + k) - p.expert_first;
       int dest = -1;
       float g = 0.0f;
       if (e >= 0 && e < p.experts_local) {
-        g = __ldg(p.gs + e);
-        dest = __ldg(p.group_offsets + e) + __ldg(p.rank + token * p.topk + k);
-        p.row_weight[dest] = __ldg(p.weights + token * p.topk + k);
+        g = ld_ordered(p.gs + e);
+        dest = ld_ordered(p.group_offsets + e) + ld_ordered(p.rank + token * p.topk + k);
+        p.row_weight[dest] = ld_ordered(p.weights + token * p.topk + k);
         p.row_token[dest] = (int)token;
       }
       s_dest[buf][k] = dest;
@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(512) moe_permute_quantize_kernel(const Permute
 // holding the token's expert outputs are looked up once, then every thread sums 8 columns at a time over those rows, in the order of the token's pairs,
 // with the loads of up to eight rows issued before the first addition.
 __global__ void __launch_bounds__(256)
-moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ ids,
-                     const int* __restrict__ rank, const int* __restrict__ group_offsets,
+moe_unpermute_kernel(const __nv_bfloat16* y, const int* ids,
+                     const int* rank, const int* group_offsets,
                      __nv_bfloat16* __restrict__ out, int tokens, int hidden, int topk,
                      int expert_first, int experts_local) {
   grid_dependency_wait();
@@ -325,8 +325,8 @@ moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict_
   const long long token = blockIdx.x;
   if ((int)threadIdx.x < topk) {
     const long long entry = token * topk + threadIdx.x;
-    const int e = __ldg(ids + entry) - expert_first;
-    s_row[threadIdx.x] = (e < 0 || e >= experts_local) ? -1 : __ldg(group_offsets + e) + __ldg(rank + entry);
+    const int e = ld_ordered(ids + entry) - expert_first;
+    s_row[threadIdx.x] = (e < 0 || e >= experts_local) ? -1 : ld_ordered(group_offsets + e) + ld_ordered(rank + entry);
   }
   __syncthreads();
   const int vecs = hidden >> 3;  // 8 bf16 per thread and step
@@ -340,7 +340,7 @@ moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict_
       for (int j = 0; j < kBatch; ++j) {
         const int row = (k0 + j < topk) ? s_row[k0 + j] : -1;
         have[j] = row >= 0;
-        if (have[j]) raw[j] = __ldg(reinterpret_cast<const uint4*>(y + (size_t)row * hidden) + vc);
+        if (have[j]) raw[j] = ld_ordered(reinterpret_cast<const uint4*>(y + (size_t)row * hidden) + vc);
       }
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {

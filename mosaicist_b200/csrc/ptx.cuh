@@ -33,6 +33,14 @@ __device__ __forceinline__ void grid_dependency_wait() {
 __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// A load behind grid_dependency_wait() of what the kernel before may have written.  It is an
+// ordinary load: __ldg (ld.global.nc) is for data that nobody writes while the kernel lives, and a
+// kernel set up under its predecessor lives while that one still writes; it may also be moved up
+// across the wait.  For the same reason such kernels take their inputs without __restrict__.
+template <class T>
+__device__ __forceinline__ T ld_ordered(const T* ptr) {
+  return *ptr;
+}
 
 // ---- mbarrier ----------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -9,6 +9,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace msc {
 
 __device__ __forceinline__ float e4m3_to_float(uint8_t b) {
@@ -201,7 +203,7 @@ __device__ __forceinline__ void load16_bf16(const __nv_bfloat16* src, float* v) 
   const uint4* s4 = reinterpret_cast<const uint4*>(src);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const uint4 raw = __ldg(s4 + i);
+    const uint4 raw = ld_ordered(s4 + i);
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

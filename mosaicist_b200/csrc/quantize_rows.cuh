@@ -65,7 +65,7 @@ __device__ __forceinline__ int owner_of_tile(const int* offsets, int l, int row0
   int count = 0;
   for (int base = 0; base < l; base += 32) {
     const int g = base + lane;
-    const bool below = g < l && __ldg(offsets + g) <= row0;
+    const bool below = g < l && ld_ordered(offsets + g) <= row0;
     count += __popc(__ballot_sync(0xffffffffu, below));
   }
   return count - 1;
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const QuantParams p)
       const uint32_t same = __ballot_sync(0xffffffffu, have && tile == t);
       if (have && tile == t && own >= 0) {
         g = own;
-        limit = __ldg(p.group_offsets + own) + __ldg(p.group_rows + own);
+        limit = ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
       }
       todo &= ~same;
     }
@@ -117,28 +117,28 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const QuantParams p)
         ok = ok && row < limit;
       } else if (p.group_rows || FMT == FMT_NVFP4) {
         gr = ok ? (int)p.m_div.div((uint32_t)row) : 0;
-        if (ok && p.group_rows) ok = row - gr * (int)p.m_div.d < __ldg(p.group_rows + gr);
+        if (ok && p.group_rows) ok = row - gr * (int)p.m_div.d < ld_ordered(p.group_rows + gr);
       }
       live[a0 + i] = ok;
       gsv[i] = 1.0f;
 #pragma unroll
       for (int w = 0; w < kWords; ++w) raw[i][w] = 0u;
       if (ok) {
-        if (FMT == FMT_NVFP4) gsv[i] = __ldg(p.gs + gr);
+        if (FMT == FMT_NVFP4) gsv[i] = ld_ordered(p.gs + gr);
         if (IN == IN_BF16) {
           const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * p.k + kb * 16);
-          *reinterpret_cast<uint4*>(&raw[i][0]) = __ldg(src);
-          *reinterpret_cast<uint4*>(&raw[i][4]) = __ldg(src + 1);
+          *reinterpret_cast<uint4*>(&raw[i][0]) = ld_ordered(src);
+          *reinterpret_cast<uint4*>(&raw[i][4]) = ld_ordered(src + 1);
         } else if (IN == IN_F32) {
           const uint4* src = reinterpret_cast<const uint4*>(static_cast<const float*>(p.x) + (size_t)row * p.k + kb * 16);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(&raw[i][4 * j]) = __ldg(src + j);
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(&raw[i][4 * j]) = ld_ordered(src + j);
         } else {
           const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * 2 * p.k + kb * 16;
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            *reinterpret_cast<uint4*>(&raw[i][4 * j]) = __ldg(reinterpret_cast<const uint4*>(base) + j);
-            *reinterpret_cast<uint4*>(&raw[i][8 + 4 * j]) = __ldg(reinterpret_cast<const uint4*>(base + p.k) + j);
+            *reinterpret_cast<uint4*>(&raw[i][4 * j]) = ld_ordered(reinterpret_cast<const uint4*>(base) + j);
+            *reinterpret_cast<uint4*>(&raw[i][8 + 4 * j]) = ld_ordered(reinterpret_cast<const uint4*>(base + p.k) + j);
           }
         }
       } else if (p.zero_out && have && row < p.rows_total) {
