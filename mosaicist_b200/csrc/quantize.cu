@@ -157,10 +157,16 @@ int msc_quantize_rows(int format, const void* x, int x_form, const float* global
                       int sf_layout, void* zero_out_bf16, int l, int rows_total, int m_stride, int k,
                       void* stream) {
   if (x_form < 0 || x_form > 2) return msc::fail(MSC_ERR_UNSUPPORTED, "x_form must be 0 (bf16), 1 (f32) or 2 (gate | up)");
-  if (!group_offsets && group_rows && m_stride <= 0)
-    return msc::fail(MSC_ERR_BAD_ARG, "group_rows without group_offsets needs m_stride");
+  if (group_offsets && !group_rows)
+    return msc::fail(MSC_ERR_BAD_ARG, "group_offsets needs group_rows");
   if (format == 0) {
-    if (!group_offsets && m_stride <= 0) return msc::fail(MSC_ERR_BAD_ARG, "m must be positive");
+    if (!group_offsets) {
+      if (m_stride <= 0) return msc::fail(MSC_ERR_BAD_ARG, "m must be positive");
+      if ((sf_layout & 1) && m_stride % 128)
+        return msc::fail(MSC_ERR_BAD_ARG, "tiled scales need m %% 128 == 0 in the masked layout");
+      if (rows_total > (long long)l * m_stride)
+        return msc::fail(MSC_ERR_BAD_ARG, "rows_total=%d exceeds l * m_stride", rows_total);
+    }
     if (zero_out_bf16 && (x_form == 2 || reinterpret_cast<uintptr_t>(zero_out_bf16) % 16))
       return msc::fail(MSC_ERR_BAD_ARG, "zero_out takes the shape of x and 16-byte alignment");
     return msc::quantize_nvfp4_rows(x, x_form == 1, global_scale, group_offsets, group_rows, q, sf, sf_layout, l,

@@ -73,6 +73,24 @@ def test_bad_arguments_are_rejected_with_a_message(lib):
     assert e.value.code == _lib.ERR_BAD_ARG
 
 
+def test_general_quantiser_refuses_what_the_named_entry_points_refuse(lib):
+    """msc_quantize_rows looks its arguments over before anything is launched: a group table without
+    row counts, tiled scales over batches that are not whole 128-row tiles, rows without a group."""
+    from mosaicist_b200 import _lib
+
+    one = ctypes.c_void_p(256)  # non-null, aligned; never dereferenced on these paths
+
+    def call(fmt=0, gs=one, offsets=None, rows=None, layout=1, l=2, total=256, m=128, k=128):
+        return lib.msc_quantize_rows(fmt, one, 0, gs, offsets, rows, one, one, layout, None, l, total, m, k, None)
+
+    for fmt in (0, 1):
+        assert call(fmt, offsets=one) == _lib.ERR_BAD_ARG and b"group_rows" in lib.msc_last_error()
+    assert call(total=192, m=96) == _lib.ERR_BAD_ARG and b"m % 128" in lib.msc_last_error()
+    assert lib.msc_nvfp4_quantize(one, 0, one, None, one, one, 1, 2, 96, 128, None) == _lib.ERR_BAD_ARG
+    assert call(total=257) == _lib.ERR_BAD_ARG and b"rows_total" in lib.msc_last_error()
+    assert call(m=0) == _lib.ERR_BAD_ARG and call(gs=None) == _lib.ERR_BAD_ARG
+
+
 def test_candidate_module_contract(monkeypatch):
     import importlib
 
