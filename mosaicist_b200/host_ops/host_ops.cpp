@@ -295,7 +295,6 @@ std::tuple<Tensor, Tensor> quantize_nvfp4(const Tensor& x, const Tensor& gs, con
   if (masked_m) need(*masked_m, "masked_m", kI32, {l});
   Tensor q = empty({l, m, k / 2}, at::kByte, x);
   Tensor sf = tiled ? empty({l, m / 128, k / 64, 32, 16}, at::kByte, x) : empty({l, m, k / 16}, at::kByte, x);
-  if (tiled && m % 128) value_error("tiled scales need m % 128 == 0 in the masked layout");
   const Lib& f = lib();
   void* st = stream();
   launch([&] {
@@ -470,7 +469,6 @@ Tensor moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf,
   need(w1_q, "w1_q", kBytes);
   need_dim(w1_q, "w1_q", 3);
   const int64_t l = hidden.size(0), m = hidden.size(1), k = hidden.size(2), n2 = w1_q.size(1), n = n2 / 2;
-  if (m % 128) value_error("tiled scales need m % 128 == 0 in the masked layout");
   need(in_gs, "global_scale", kF32, {l});
   need(masked_m, "masked_m", kI32, {l});
   need(w1_q, "w1_q", kBytes, {l, n2, k / 2});

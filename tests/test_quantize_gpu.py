@@ -61,6 +61,20 @@ def test_quantize_skips_masked_rows():
     assert np.array_equal(sfh[1, :7], O.e4m3_bytes(want_sf)[1, :7]) and not sfh[1, 7:].any()
 
 
+@pytest.mark.parametrize("silu", [False, True])
+def test_ragged_tiles_are_refused_by_the_library(silu):
+    """Tiled scales need whole 128-row tiles: the status comes from the library as its own error."""
+    from mosaicist_b200 import _lib, ops
+
+    x = torch.zeros((2, 96, 256), dtype=torch.bfloat16, device="cuda")
+    call = ops.silu_mul_quantize_nvfp4 if silu else ops.quantize_nvfp4
+    with pytest.raises(_lib.MscError) as e:
+        call(x, torch.ones(2, device="cuda"))
+    assert e.value.code == _lib.ERR_BAD_ARG
+    q, sf = call(x, torch.ones(2, device="cuda"), tiled_scales=False)      # row-major scales take any m
+    assert tuple(q.shape) == (2, 96, q.shape[2]) and not sf.any()
+
+
 def test_silu_mul_quantize_matches_oracle():
     """The activation goes through expf on the device and np.exp on the host, so allow the
     rare block whose rounding flips; at least 99.9 % of bytes must be identical and every
