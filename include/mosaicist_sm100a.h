@@ -159,7 +159,8 @@ int msc_moe_masked(const void* hidden, const void* w1_q, const void* w1_sf, cons
 /* The general row quantiser; the named entry points below are special cases of it.
  *   format 0 NVFP4, 1 MXFP8; x_form 0 bf16, 1 fp32, 2 (NVFP4 only) bf16 gate | up of width 2k,
  *   quantised as silu(gate) * up; global_scale (l) for NVFP4;
- *   group_offsets (l) ascending multiples of 128 with group_rows (l), or NULL: group g owns rows
+ *   group_offsets (l) ascending with group_rows (l) (any offsets here; the GEMMs want multiples of
+ *   128), or NULL: group g owns rows
  *   [g * m_stride, + group_rows[g]) (group_rows NULL: all of them);
  *   zero_out_bf16 (rows_total, k) or NULL: rows that are not live are set to zero there, so a
  *   caller whose result has the shape of x needs no separate clearing pass. */

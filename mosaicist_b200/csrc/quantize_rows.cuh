@@ -7,7 +7,7 @@
 // (MXFP8) instead of 4-byte words 512 bytes apart, each of which costs an L2 transaction of its
 // own.  The loads of the four rows are issued before anything is computed; a warp reads 1 KB of
 // a row at a time.  Which rows are live is a property of the quad (its 128-row tile lies in one
-// ragged group) or of the row (masked batches), and the index arithmetic of the four blocks is
+// ragged group, unless a group starts inside it) or of the row (masked batches), and the index arithmetic of the four blocks is
 // shared: multiplications by precomputed reciprocals instead of 64-bit divisions.
 //
 // Bound by HBM for MXFP8 and by a mix of issue slots and HBM for NVFP4.  Cold, 16384 x 7168,
@@ -44,7 +44,7 @@ struct QuantParams {
   const void* x;            // (rows_total, k) or, with IN_SILU, (rows_total, 2k) gate | up
   const float* gs;          // (l) per-group global scale (NVFP4)
   const int* group_rows;    // (l) or null: rows at or beyond it are not live
-  const int* group_offsets; // (l) ascending multiples of 128, or null: group g starts at g * m_stride
+  const int* group_offsets; // (l) ascending, or null: group g starts at g * m_stride
   uint8_t* q;               // (rows_total, k/2) e2m1 pairs or (rows_total, k) e4m3
   uint8_t* sf;              // tiled or row-major scale bytes
   __nv_bfloat16* zero_out;  // (rows_total, k) or null: rows that are not live are set to zero here
@@ -57,22 +57,35 @@ struct QuantParams {
   FastDiv m_div;            // by m_stride (masked layout)
 };
 
-// Owner of the 128-row tile that starts at `row0` in the ragged layout: the last group whose
-// offset is <= row0 (offsets ascend; an empty group shares the offset of the group after it).
-// The lanes of a converged warp ask about the same row and each compares every 32nd offset.
-__device__ __forceinline__ int owner_of_tile(const int* offsets, int l, int row0) {
+// Owner of row `row0` in the ragged layout: the last group whose offset is <= row0 (offsets ascend; an
+// empty group shares the offset of the group after it); -1 before the first group.  Also says whether
+// a group starts inside the 127 rows after it.  The lanes of a converged warp ask about the same row
+// and each compares every 32nd offset.
+__device__ __forceinline__ int owner_of_tile(const int* offsets, int l, int row0, bool& shared) {
   const int lane = threadIdx.x & 31;
-  int count = 0;
+  int count = 0, upto = 0;
   for (int base = 0; base < l; base += 32) {
     const int g = base + lane;
-    const bool below = g < l && ld_ordered(offsets + g) <= row0;
-    count += __popc(__ballot_sync(0xffffffffu, below));
+    const int off = g < l ? ld_ordered(offsets + g) : 0x7fffffff;
+    count += __popc(__ballot_sync(0xffffffffu, off <= row0));
+    upto += __popc(__ballot_sync(0xffffffffu, off <= row0 + 127));
   }
+  shared = upto != count;
   return count - 1;
 }
+// The same for one thread's row.
+__device__ __forceinline__ int owner_of_row(const int* offsets, int l, int row) {
+  int lo = -1, hi = l - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (ld_ordered(offsets + mid) <= row) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
 
+// (five blocks of the bf16 -> MXFP8 form fit an SM at 48 registers; the others have four)
 template <int FMT, int IN>
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4) quantize_rows_kernel(const QuantParams p) {
   grid_dependency_wait();
   grid_launch_dependents();
   const uint32_t unit = blockIdx.x * 256u + threadIdx.x;
@@ -83,48 +96,69 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const QuantParams p)
   const int tile = (int)(quad >> 5), b = (int)(quad & 31u);
   const int row_b = tile * 128 + b;         // row of a = 0
 
-  int g = 0, limit = 0;                     // ragged: live rows are [.., limit)
+  // Which of the four rows are live, and their global scales.  Ragged: the owner of the tile holds all
+  // of them.  The GEMMs want groups at multiples of 128; the quantisers alone take any ascending
+  // offsets, so where a group starts inside the tile each row looks its own group up.
+  bool live[4];
+  float gsv[4];
   if (p.group_offsets) {
+    int g = 0, limit = 0;
+    bool shared = false;
     // a warp spans at most two tiles when a row has 32 blocks or more; short rows take more steps
     uint32_t todo = __ballot_sync(0xffffffffu, have);
     while (todo) {
       const int lead = __ffs(todo) - 1;
       const int t = __shfl_sync(0xffffffffu, tile, lead);
-      const int own = owner_of_tile(p.group_offsets, p.l, t * 128);
+      bool inside;
+      const int own = owner_of_tile(p.group_offsets, p.l, t * 128, inside);
       const uint32_t same = __ballot_sync(0xffffffffu, have && tile == t);
-      if (have && tile == t && own >= 0) {
-        g = own;
-        limit = ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
+      if (have && tile == t) {
+        shared = inside;
+        if (own >= 0) {
+          g = own;
+          limit = ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
+        }
       }
       todo &= ~same;
+    }
+    const float gs = FMT == FMT_NVFP4 && have ? ld_ordered(p.gs + g) : 1.0f;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int row = row_b + 32 * a;
+      live[a] = have && row < p.rows_total && row < limit;
+      gsv[a] = gs;
+      if (shared && row < p.rows_total) {
+        const int own = owner_of_row(p.group_offsets, p.l, row);
+        live[a] = own >= 0 && row < ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
+        if (FMT == FMT_NVFP4 && live[a]) gsv[a] = ld_ordered(p.gs + own);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int row = row_b + 32 * a;
+      live[a] = have && row < p.rows_total;
+      gsv[a] = 1.0f;
+      if (FMT == FMT_NVFP4 && live[a]) {
+        const int g = (int)p.m_div.div((uint32_t)row);
+        gsv[a] = ld_ordered(p.gs + g);
+        if (p.group_rows) live[a] = row - g * (int)p.m_div.d < ld_ordered(p.group_rows + g);
+      }
     }
   }
 
   constexpr int kWords = IN == IN_BF16 ? 8 : 16;   // 32-bit words of input per block
   constexpr int kAhead = IN == IN_BF16 ? 4 : 2;    // rows whose loads are issued together
   uint32_t words[4];                               // scale word of each row, after pooling
-  bool live[4];
 #pragma unroll
   for (int a0 = 0; a0 < 4; a0 += kAhead) {
     uint32_t raw[kAhead][kWords];
-    float gsv[kAhead];
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       const int row = row_b + 32 * (a0 + i);
-      bool ok = have && row < p.rows_total;
-      int gr = g;
-      if (p.group_offsets) {
-        ok = ok && row < limit;
-      } else if (p.group_rows || FMT == FMT_NVFP4) {
-        gr = ok ? (int)p.m_div.div((uint32_t)row) : 0;
-        if (ok && p.group_rows) ok = row - gr * (int)p.m_div.d < ld_ordered(p.group_rows + gr);
-      }
-      live[a0 + i] = ok;
-      gsv[i] = 1.0f;
 #pragma unroll
       for (int w = 0; w < kWords; ++w) raw[i][w] = 0u;
-      if (ok) {
-        if (FMT == FMT_NVFP4) gsv[i] = ld_ordered(p.gs + gr);
+      if (live[a0 + i]) {
         if (IN == IN_BF16) {
           const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * p.k + kb * 16);
           *reinterpret_cast<uint4*>(&raw[i][0]) = ld_ordered(src);
@@ -172,7 +206,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const QuantParams p)
       if (FMT == FMT_NVFP4) {
         uint2 q8 = make_uint2(0u, 0u);
         if (live[a]) {
-          quantize_16_amax(v, amax, gsv[i], q8, sfb);
+          quantize_16_amax(v, amax, gsv[a], q8, sfb);
           *reinterpret_cast<uint2*>(p.q + (size_t)row * (p.k >> 1) + kb * 8) = q8;
         }
         words[a] = gather_scale_word(sfb);          // lanes 0 mod 4: bytes of four blocks

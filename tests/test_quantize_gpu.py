@@ -200,6 +200,61 @@ def test_mxfp8_quantize_ragged_skips_rows_outside_groups():
     assert np.array_equal(sf_rows[live], want_sf[live]) and (sf_rows[~live] == 0xEE).all()
 
 
+# groups that start anywhere: inside a tile, several in one tile, empty ones, a first one not at row 0,
+# more groups than a warp's lanes; (row counts, gap before each group)
+_LOOSE = [([100, 0, 130, 1], [0, 3, 0, 40]), ([5] * 70, [2] * 70), ([0, 200], [77, 51]), ([128, 128, 3], [0, 0, 0])]
+
+
+@pytest.mark.parametrize("rows_list,gaps", _LOOSE)
+@pytest.mark.parametrize("form", ["mxfp8", "nvfp4", "nvfp4_silu"])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_ragged_quantisers_take_any_ascending_offsets(rows_list, gaps, form, dtype):
+    """Only the GEMMs need groups at multiples of 128: the quantisers write the rows inside a group and
+    no others, wherever the groups start."""
+    from mosaicist_b200 import ops
+    from oracle import mxfp8 as X
+
+    if form == "nvfp4_silu" and dtype == "f32":
+        pytest.skip("the fused form takes bf16")
+    k, offs, at = 128, [], 0
+    for r, gap in zip(rows_list, gaps):
+        offs.append(at + gap)
+        at += gap + r
+    tot = at + 9
+    live = np.zeros(tot, bool)
+    for o, r in zip(offs, rows_list):
+        live[o:o + r] = True
+    o_t, r_t = T(np.array(offs, np.int32)), T(np.array(rows_list, np.int32))
+    x = np.random.default_rng([6, tot]).standard_normal((tot, 2 * k if form == "nvfp4_silu" else k)).astype(np.float32)
+    if dtype == "bf16":
+        x = x.astype(ml_dtypes.bfloat16).astype(np.float32)
+    xt = T(x).to(torch.bfloat16) if dtype == "bf16" else T(x)
+    per_sf = 32 if form == "mxfp8" else 16
+    q = torch.full((tot, k if form == "mxfp8" else k // 2), 0xEE, dtype=torch.uint8, device="cuda")
+    sf = torch.full(((tot + 127) // 128, k // (4 * per_sf), 32, 16), 0xEE, dtype=torch.uint8, device="cuda")
+    if form == "mxfp8":
+        want_q, want_sf = X.quantize_mxfp8(x)
+        want_q = want_q.view(np.uint8)
+        ops.quantize_mxfp8(xt, True, o_t, r_t, out=(q, sf))
+    else:
+        gs = np.linspace(100.0, 900.0, len(rows_list)).astype(np.float32)
+        silu = form == "nvfp4_silu"
+        ops.quantize_nvfp4_ragged(xt, T(gs), o_t, r_t, silu, out=(q, sf))
+        want_q, want_sf = np.zeros((tot, k // 2), np.uint8), np.zeros((tot, k // 16), np.uint8)
+        for g, (o, r) in enumerate(zip(offs, rows_list)):
+            if r and silu:      # the oracle's exponential is another one: the masked form of the same kernel is exact
+                pad = torch.zeros((1, 512, 2 * k), dtype=torch.bfloat16, device="cuda")
+                pad[0, :r] = xt[o:o + r]
+                a_q, a_sf = ops.silu_mul_quantize_nvfp4(pad, T(gs[g:g + 1]), None, tiled_scales=False)
+                want_q[o:o + r], want_sf[o:o + r] = a_q[0, :r].cpu().numpy(), a_sf[0, :r].cpu().numpy()
+            elif r:
+                a_q, a_sf = O.quantize_nvfp4(x[None, o:o + r], gs[g:g + 1])
+                want_q[o:o + r], want_sf[o:o + r] = O.pack_e2m1(a_q)[0], O.e4m3_bytes(a_sf)[0]
+    qh, sfh = q.cpu().numpy(), O.from_mma_scale_layout(sf.cpu().numpy(), tot)
+    assert np.array_equal(qh[live], want_q[live]) and (qh[~live] == 0xEE).all()
+    assert np.array_equal(sfh[live], want_sf[live]) and (sfh[~live] == 0xEE).all()
+
+
 @pytest.mark.parametrize("shape", [(3, 128, 256), (8, 512, 2048), (1, 8, 8)])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_global_scale_matches_oracle(shape, dtype):
