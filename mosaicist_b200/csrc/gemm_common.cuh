@@ -137,12 +137,14 @@ struct TileCursor {
     while (true) {
       if (!primed) {
         if (g >= p.l) return false;
-        // every lane reads the same word; the broadcast tells the compiler so
-        rows = p.group_rows ? __shfl_sync(0xffffffffu, ld_ordered(p.group_rows + g), 0) : p.m_stride;
+        // every lane reads the same words, both loads under way before either is waited for; the
+        // broadcasts tell the compiler that all lanes agree
+        const int r = p.group_rows ? ld_ordered(p.group_rows + g) : p.m_stride;
+        const int o = p.group_offsets ? ld_ordered(p.group_offsets + g) : g * p.m_stride;
+        rows = __shfl_sync(0xffffffffu, r, 0);
+        off = __shfl_sync(0xffffffffu, o, 0);
         if (rows < 0) rows = 0;
         if (p.m_stride > 0 && rows > p.m_stride) rows = p.m_stride;
-        off = p.group_offsets ? __shfl_sync(0xffffffffu, ld_ordered(p.group_offsets + g), 0)
-                              : g * p.m_stride;
         // a group table that reaches beyond the buffers (an overflowing expert-parallel step,
         // a stale table after a timed-out wait) is cut to what the buffers hold
         if (off < 0 || off >= p.rows_total) rows = 0;

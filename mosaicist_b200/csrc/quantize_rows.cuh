@@ -83,9 +83,117 @@ __device__ __forceinline__ int owner_of_row(const int* offsets, int l, int row) 
   return lo;
 }
 
-// (five blocks of the bf16 -> MXFP8 form fit an SM at 48 registers; the others have four)
+template <int IN>
+constexpr int kInWords = IN == IN_BF16 ? 8 : 16;   // 32-bit words of input per block of 16
+
+template <int IN>
+__device__ __forceinline__ void load_block(const QuantParams& p, int row, int kb, uint32_t* raw) {
+  if (IN == IN_BF16) {
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * p.k + kb * 16);
+    *reinterpret_cast<uint4*>(raw) = ld_ordered(src);
+    *reinterpret_cast<uint4*>(raw + 4) = ld_ordered(src + 1);
+  } else if (IN == IN_F32) {
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const float*>(p.x) + (size_t)row * p.k + kb * 16);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(raw + 4 * j) = ld_ordered(src + j);
+  } else {
+    const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * 2 * p.k + kb * 16;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      *reinterpret_cast<uint4*>(raw + 4 * j) = ld_ordered(reinterpret_cast<const uint4*>(base) + j);
+      *reinterpret_cast<uint4*>(raw + 8 + 4 * j) = ld_ordered(reinterpret_cast<const uint4*>(base + p.k) + j);
+    }
+  }
+}
+
+// Quantises a block and stores its values if its row is live.  Made by whole warps: returns the scale
+// word of the row, valid in lanes 0 mod 4 (NVFP4) or 0 mod 8 (MXFP8), zero bytes where not live.
 template <int FMT, int IN>
-__global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4) quantize_rows_kernel(const QuantParams p) {
+__device__ __forceinline__ uint32_t quantize_block(const QuantParams& p, int row, int kb, uint32_t* raw, bool live, float gs) {
+  float v[16];
+  float amax;
+  if (IN == IN_BF16) {
+    amax = amax_bf16x16(raw);
+    unpack_bf16x16(raw, v);
+  } else if (IN == IN_F32) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(raw[e]);
+    amax = amax_f32x16(v);
+  } else {
+    // row holds [gate (k) | up (k)] in bf16; the activation stays fp32 (nvfp4.py:81-88)
+    float up[16];
+    unpack_bf16x16(raw, v);
+    unpack_bf16x16(raw + 8, up);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = silu_mul(v[e], up[e]);
+    amax = amax_f32x16(v);
+  }
+  uint32_t sfb = 0;
+  if (FMT == FMT_NVFP4) {
+    uint2 q8 = make_uint2(0u, 0u);
+    if (live) {
+      quantize_16_amax(v, amax, gs, q8, sfb);
+      *reinterpret_cast<uint2*>(p.q + (size_t)row * (p.k >> 1) + kb * 8) = q8;
+    }
+    return gather_scale_word(sfb);              // lanes 0 mod 4: bytes of four blocks
+  }
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // two lanes share a block of 32
+  if (live) {
+    sfb = mx_scale_byte(amax);
+    const uint4 q16 = mx_pack_16(v, sfb);
+    uint8_t* dst = p.q + (size_t)row * p.k + kb * 16;
+    if (p.wide & 2) {
+      *reinterpret_cast<uint4*>(dst) = q16;
+    } else {
+      reinterpret_cast<uint2*>(dst)[0] = make_uint2(q16.x, q16.y);
+      reinterpret_cast<uint2*>(dst)[1] = make_uint2(q16.z, q16.w);
+    }
+  }
+  uint32_t w = sfb;                             // lanes 0 mod 8: bytes of four blocks
+  w |= __shfl_down_sync(0xffffffffu, sfb, 2) << 8;
+  w |= __shfl_down_sync(0xffffffffu, sfb, 4) << 16;
+  w |= __shfl_down_sync(0xffffffffu, sfb, 6) << 24;
+  return w;
+}
+template <int FMT>
+constexpr int kScaleLanes = FMT == FMT_NVFP4 ? 4 : 8;   // lanes (blocks of 16) per scale word
+
+// The blocks of a warp that meets a tile inside which a group starts: the GEMMs want groups at
+// multiples of 128, the quantisers alone take any ascending offsets.  One row at a time, each with
+// its own group.  Out of line, so that it costs the kernel no registers.
+template <int FMT, int IN>
+__device__ __noinline__ void quantize_shared_tiles(const QuantParams& p, int row_b, int kb, bool have) {
+#pragma unroll 1
+  for (int a = 0; a < 4; ++a) {
+    const int row = row_b + 32 * a;
+    bool live = have && row < p.rows_total;
+    float gs = 1.0f;
+    if (live) {
+      const int own = owner_of_row(p.group_offsets, p.l, row);
+      live = own >= 0 && row < ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
+      if (FMT == FMT_NVFP4 && live) gs = ld_ordered(p.gs + own);
+    }
+    uint32_t raw[kInWords<IN>];
+#pragma unroll
+    for (int w = 0; w < kInWords<IN>; ++w) raw[w] = 0u;
+    if (live) load_block<IN>(p, row, kb, raw);
+    if (p.zero_out && have && !live && row < p.rows_total) {
+      uint4* dst = reinterpret_cast<uint4*>(p.zero_out + (size_t)row * p.k + kb * 16);
+      dst[0] = dst[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    const uint32_t word = quantize_block<FMT, IN>(p, row, kb, raw, live, gs);
+    if (!have || (kb & (kScaleLanes<FMT> - 1))) continue;
+    const int kw = kb / kScaleLanes<FMT>, kwords = (p.k >> 4) / kScaleLanes<FMT>;
+    if (p.tiled) {
+      if (live || p.zero_rest) *reinterpret_cast<uint32_t*>(p.sf + tiled_sf_word(row, kw, kwords)) = word;
+    } else if (live || (p.zero_rest && row < p.rows_total)) {
+      *reinterpret_cast<uint32_t*>(p.sf + ((size_t)row * kwords + kw) * 4) = word;
+    }
+  }
+}
+
+template <int FMT, int IN, bool RAGGED>
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const __grid_constant__ QuantParams p) {
   grid_dependency_wait();
   grid_launch_dependents();
   const uint32_t unit = blockIdx.x * 256u + threadIdx.x;
@@ -96,12 +204,10 @@ __global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4
   const int tile = (int)(quad >> 5), b = (int)(quad & 31u);
   const int row_b = tile * 128 + b;         // row of a = 0
 
-  // Which of the four rows are live, and their global scales.  Ragged: the owner of the tile holds all
-  // of them.  The GEMMs want groups at multiples of 128; the quantisers alone take any ascending
-  // offsets, so where a group starts inside the tile each row looks its own group up.
+  // which of the four rows are live, and their global scales
   bool live[4];
   float gsv[4];
-  if (p.group_offsets) {
+  if (RAGGED) {
     int g = 0, limit = 0;
     bool shared = false;
     // a warp spans at most two tiles when a row has 32 blocks or more; short rows take more steps
@@ -111,15 +217,17 @@ __global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4
       const int t = __shfl_sync(0xffffffffu, tile, lead);
       bool inside;
       const int own = owner_of_tile(p.group_offsets, p.l, t * 128, inside);
+      shared = shared || inside;
       const uint32_t same = __ballot_sync(0xffffffffu, have && tile == t);
-      if (have && tile == t) {
-        shared = inside;
-        if (own >= 0) {
-          g = own;
-          limit = ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
-        }
+      if (have && tile == t && own >= 0) {
+        g = own;
+        limit = ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
       }
       todo &= ~same;
+    }
+    if (shared) {                           // the same for the whole warp
+      quantize_shared_tiles<FMT, IN>(p, row_b, kb, have);
+      return;
     }
     const float gs = FMT == FMT_NVFP4 && have ? ld_ordered(p.gs + g) : 1.0f;
 #pragma unroll
@@ -127,11 +235,6 @@ __global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4
       const int row = row_b + 32 * a;
       live[a] = have && row < p.rows_total && row < limit;
       gsv[a] = gs;
-      if (shared && row < p.rows_total) {
-        const int own = owner_of_row(p.group_offsets, p.l, row);
-        live[a] = own >= 0 && row < ld_ordered(p.group_offsets + own) + ld_ordered(p.group_rows + own);
-        if (FMT == FMT_NVFP4 && live[a]) gsv[a] = ld_ordered(p.gs + own);
-      }
     }
   } else {
 #pragma unroll
@@ -147,93 +250,29 @@ __global__ void __launch_bounds__(256, FMT == FMT_MXFP8 && IN == IN_BF16 ? 5 : 4
     }
   }
 
-  constexpr int kWords = IN == IN_BF16 ? 8 : 16;   // 32-bit words of input per block
   constexpr int kAhead = IN == IN_BF16 ? 4 : 2;    // rows whose loads are issued together
-  uint32_t words[4];                               // scale word of each row, after pooling
+  uint32_t words[4];                               // scale word of each row
 #pragma unroll
   for (int a0 = 0; a0 < 4; a0 += kAhead) {
-    uint32_t raw[kAhead][kWords];
+    uint32_t raw[kAhead][kInWords<IN>];
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       const int row = row_b + 32 * (a0 + i);
 #pragma unroll
-      for (int w = 0; w < kWords; ++w) raw[i][w] = 0u;
+      for (int w = 0; w < kInWords<IN>; ++w) raw[i][w] = 0u;
       if (live[a0 + i]) {
-        if (IN == IN_BF16) {
-          const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * p.k + kb * 16);
-          *reinterpret_cast<uint4*>(&raw[i][0]) = ld_ordered(src);
-          *reinterpret_cast<uint4*>(&raw[i][4]) = ld_ordered(src + 1);
-        } else if (IN == IN_F32) {
-          const uint4* src = reinterpret_cast<const uint4*>(static_cast<const float*>(p.x) + (size_t)row * p.k + kb * 16);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(&raw[i][4 * j]) = ld_ordered(src + j);
-        } else {
-          const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(p.x) + (size_t)row * 2 * p.k + kb * 16;
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            *reinterpret_cast<uint4*>(&raw[i][4 * j]) = ld_ordered(reinterpret_cast<const uint4*>(base) + j);
-            *reinterpret_cast<uint4*>(&raw[i][8 + 4 * j]) = ld_ordered(reinterpret_cast<const uint4*>(base + p.k) + j);
-          }
-        }
+        load_block<IN>(p, row, kb, raw[i]);
       } else if (p.zero_out && have && row < p.rows_total) {
         uint4* dst = reinterpret_cast<uint4*>(p.zero_out + (size_t)row * p.k + kb * 16);
         dst[0] = dst[1] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
 #pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
-      const int a = a0 + i;
-      const int row = row_b + 32 * a;
-      float v[16];
-      float amax;
-      if (IN == IN_BF16) {
-        amax = amax_bf16x16(raw[i]);
-        unpack_bf16x16(raw[i], v);
-      } else if (IN == IN_F32) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(raw[i][e]);
-        amax = amax_f32x16(v);
-      } else {
-        // row holds [gate (k) | up (k)] in bf16; the activation stays fp32 (nvfp4.py:81-88)
-        float up[16];
-        unpack_bf16x16(raw[i], v);
-        unpack_bf16x16(raw[i] + 8, up);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = silu_mul(v[e], up[e]);
-        amax = amax_f32x16(v);
-      }
-      uint32_t sfb = 0;
-      if (FMT == FMT_NVFP4) {
-        uint2 q8 = make_uint2(0u, 0u);
-        if (live[a]) {
-          quantize_16_amax(v, amax, gsv[a], q8, sfb);
-          *reinterpret_cast<uint2*>(p.q + (size_t)row * (p.k >> 1) + kb * 8) = q8;
-        }
-        words[a] = gather_scale_word(sfb);          // lanes 0 mod 4: bytes of four blocks
-      } else {
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // two lanes share a block of 32
-        if (live[a]) {
-          sfb = mx_scale_byte(amax);
-          const uint4 q16 = mx_pack_16(v, sfb);
-          uint8_t* dst = p.q + (size_t)row * p.k + kb * 16;
-          if (p.wide & 2) {
-            *reinterpret_cast<uint4*>(dst) = q16;
-          } else {
-            reinterpret_cast<uint2*>(dst)[0] = make_uint2(q16.x, q16.y);
-            reinterpret_cast<uint2*>(dst)[1] = make_uint2(q16.z, q16.w);
-          }
-        }
-        uint32_t w = sfb;                            // lanes 0 mod 8: bytes of four blocks
-        w |= __shfl_down_sync(0xffffffffu, sfb, 2) << 8;
-        w |= __shfl_down_sync(0xffffffffu, sfb, 4) << 16;
-        w |= __shfl_down_sync(0xffffffffu, sfb, 6) << 24;
-        words[a] = w;
-      }
-    }
+    for (int i = 0; i < kAhead; ++i)
+      words[a0 + i] = quantize_block<FMT, IN>(p, row_b + 32 * (a0 + i), kb, raw[i], live[a0 + i], gsv[a0 + i]);
   }
-  constexpr int kLanes = FMT == FMT_NVFP4 ? 4 : 8;   // lanes (blocks of 16) per scale word
-  if (!have || (kb & (kLanes - 1))) return;
-  const int kw = kb / kLanes, kwords = kblocks / kLanes;
+  if (!have || (kb & (kScaleLanes<FMT> - 1))) return;
+  const int kw = kb / kScaleLanes<FMT>, kwords = kblocks / kScaleLanes<FMT>;
   if (p.tiled) {
     uint8_t* dst = p.sf + tiled_sf_word(row_b, kw, kwords);
     const bool all = p.zero_rest || (live[0] && live[1] && live[2] && live[3]);   // dead rows' words are 0
@@ -267,9 +306,14 @@ int launch_quantize_rows(QuantParams& p, int in_form, int m_stride, cudaStream_t
   p.m_div = FastDiv::make((uint32_t)(m_stride > 0 ? m_stride : 1));
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t lc = pdl_launch_config((int)((units + 255) / 256), 256, 0, stream, attr);
-  if (in_form == IN_BF16) MSC_CUDA_OK(cudaLaunchKernelEx(&lc, quantize_rows_kernel<FMT, IN_BF16>, p));
-  else if (in_form == IN_F32) MSC_CUDA_OK(cudaLaunchKernelEx(&lc, quantize_rows_kernel<FMT, IN_F32>, p));
-  else if constexpr (FMT == FMT_NVFP4) MSC_CUDA_OK(cudaLaunchKernelEx(&lc, quantize_rows_kernel<FMT, IN_SILU>, p));
+  const bool ragged = p.group_offsets != nullptr;
+  auto launch = [&](auto kern) { return cudaLaunchKernelEx(&lc, kern, p); };
+  if (in_form == IN_BF16)
+    MSC_CUDA_OK(ragged ? launch(quantize_rows_kernel<FMT, IN_BF16, true>) : launch(quantize_rows_kernel<FMT, IN_BF16, false>));
+  else if (in_form == IN_F32)
+    MSC_CUDA_OK(ragged ? launch(quantize_rows_kernel<FMT, IN_F32, true>) : launch(quantize_rows_kernel<FMT, IN_F32, false>));
+  else if constexpr (FMT == FMT_NVFP4)
+    MSC_CUDA_OK(ragged ? launch(quantize_rows_kernel<FMT, IN_SILU, true>) : launch(quantize_rows_kernel<FMT, IN_SILU, false>));
   return MSC_OK;
 }
 
