@@ -459,16 +459,28 @@ Tensor gemm_int4_ragged(const Tensor& a, const Tensor& b_q, const Tensor& scales
   return *out;
 }
 
-// The masked MoE layer; zero_rest: rows at or beyond masked_m come back as zeros.
-Tensor moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf, const Tensor& w1_gs, const Tensor& w1_alpha,
-                  const Tensor& w2_q, const Tensor& w2_sf, const Tensor& w2_gs, const Tensor& w2_alpha,
-                  const Tensor& masked_m, const Tensor& in_gs, const Tensor& a2_gs, const OptTensor& g1_alpha,
-                  const OptTensor& g2_alpha, bool zero_rest) {
-  need(hidden, "x", kBf16);
-  need_dim(hidden, "x", 3);
-  need(w1_q, "w1_q", kBytes);
-  need_dim(w1_q, "w1_q", 3);
+// Whether a factor of the masked layer is what msc_moe_masked reads: one fp32 per expert.
+bool per_expert(const OptTensor& t, int64_t l) {
+  return t && t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->dim() == 1 && t->size(0) == l;
+}
+
+// The masked MoE layer in one call; zero_rest: rows at or beyond masked_m come back as zeros.  Nothing
+// is returned for the forms that only the layer's separate steps take (mosaicist_b200.moe): fp32
+// activations, global scales and alphas that have to be broadcast, converted or copied first, a
+// second weight whose rows are not hidden's columns, sizes the fused call is not built for.
+OptTensor moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf, const OptTensor& w1_gs, const OptTensor& w1_alpha,
+                     const Tensor& w2_q, const Tensor& w2_sf, const OptTensor& w2_gs, const OptTensor& w2_alpha,
+                     const Tensor& masked_m, const Tensor& in_gs, const Tensor& a2_gs, const OptTensor& g1_alpha,
+                     const OptTensor& g2_alpha, bool zero_rest) {
+  if (hidden.scalar_type() != at::kBFloat16 || hidden.dim() != 3 || w1_q.dim() != 3 || w2_q.dim() != 3) return std::nullopt;
   const int64_t l = hidden.size(0), m = hidden.size(1), k = hidden.size(2), n2 = w1_q.size(1), n = n2 / 2;
+  if (m % 128 || k % 128 || n % 64 || w2_q.size(1) != k) return std::nullopt;
+  if (g1_alpha || g2_alpha) {
+    if (!per_expert(g1_alpha, l) || !per_expert(g2_alpha, l)) return std::nullopt;
+  } else if (!per_expert(w1_gs, l) || !per_expert(w1_alpha, l) || !per_expert(w2_gs, l) || !per_expert(w2_alpha, l)) {
+    return std::nullopt;
+  }
+  need(hidden, "x", kBf16);
   need(in_gs, "global_scale", kF32, {l});
   need(masked_m, "masked_m", kI32, {l});
   need(w1_q, "w1_q", kBytes, {l, n2, k / 2});
@@ -476,15 +488,6 @@ Tensor moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf,
   need(w2_q, "b_q", kBytes, {l, k, n / 2});
   need(w2_sf, "b_sf", kBytes, {l, k / 128, n / 64, 32, 16});
   need(a2_gs, "out_global_scale", kF32, {l});
-  if (g1_alpha) {
-    need(*g1_alpha, "alpha", kF32, {l});
-    need(*g2_alpha, "alpha", kF32, {l});
-  } else {
-    need(w1_gs, "w1_gs", kF32, {l});
-    need(w1_alpha, "w1_alpha", kF32, {l});
-    need(w2_gs, "w2_gs", kF32, {l});
-    need(w2_alpha, "w2_alpha", kF32, {l});
-  }
   const Lib& f = lib();
   const size_t bytes = f.msc_moe_masked_workspace(l, m, k, n);
   Tensor ws = empty({(int64_t)bytes}, at::kByte, hidden);
@@ -497,6 +500,30 @@ Tensor moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf,
                             out.data_ptr(), zero_rest ? 1 : 0, l, m, k, n, st);
   });
   return out;
+}
+
+// The layer's separate steps, written in Python: the torch operator's way for what moe_masked leaves.
+Tensor moe_masked_steps(std::initializer_list<Tensor> args) {
+  Gil gil;
+  PyObject* mod = PyImport_ImportModule("mosaicist_b200.moe");
+  PyObject* fn = mod ? PyObject_GetAttrString(mod, "moe_masked_steps") : nullptr;
+  Py_XDECREF(mod);
+  PyObject* tuple = fn ? PyTuple_New(args.size()) : nullptr;
+  Py_ssize_t i = 0;
+  bool ok = tuple != nullptr;
+  for (const Tensor& t : args) {
+    if (!ok) break;
+    PyObject* o = THPVariable_Wrap(t);
+    ok = o != nullptr;
+    if (ok) PyTuple_SET_ITEM(tuple, i++, o);
+  }
+  PyObject* out = ok ? PyObject_CallObject(fn, tuple) : nullptr;
+  Py_XDECREF(tuple);
+  Py_XDECREF(fn);
+  if (!out) raise();
+  const Tensor result = THPVariable_Unpack(out);
+  Py_DECREF(out);
+  return result;
 }
 
 // ---- the CPython module ------------------------------------------------------------------------
@@ -631,12 +658,15 @@ PY_FUNCTION(mixed_grouped_gemm_int4, 11) {
                                tensor(a[4], "group_rows"), opt_tensor(a[5], "alpha"), integer(a[6]), opt_tensor(a[7], "workspace"),
                                opt_tensor(a[8], "out"), a[9] == Py_None ? -1 : (int)truth(a[9]), (int)integer(a[10])));
 }
+// -> the result, or None where the separate steps have to be taken
 PY_FUNCTION(moe_masked, 14) {
-  return wrap(moe_masked(tensor(a[0], "x"), tensor(a[1], "w1_q"), tensor(a[2], "w1_sf"), tensor(a[3], "w1_gs"),
-                         tensor(a[4], "w1_alpha"), tensor(a[5], "w2_q"), tensor(a[6], "w2_sf"), tensor(a[7], "w2_gs"),
-                         tensor(a[8], "w2_alpha"), tensor(a[9], "masked_m"), tensor(a[10], "global_scale"),
-                         tensor(a[11], "a2_global_scale"), opt_tensor(a[12], "folded alpha"), opt_tensor(a[13], "folded alpha"),
-                         false));
+  const OptTensor out =
+      moe_masked(tensor(a[0], "x"), tensor(a[1], "w1_q"), tensor(a[2], "w1_sf"), opt_tensor(a[3], "w1_gs"),
+                 opt_tensor(a[4], "w1_alpha"), tensor(a[5], "w2_q"), tensor(a[6], "w2_sf"), opt_tensor(a[7], "w2_gs"),
+                 opt_tensor(a[8], "w2_alpha"), tensor(a[9], "masked_m"), tensor(a[10], "global_scale"),
+                 tensor(a[11], "a2_global_scale"), opt_tensor(a[12], "folded alpha"), opt_tensor(a[13], "folded alpha"), false);
+  if (out) return wrap(*out);
+  Py_RETURN_NONE;
 }
 
 // ---- the routed layer (mosaicist_b200.moe.MegaMoE) ----------------------------------------------
@@ -794,8 +824,12 @@ Tensor op_grouped_gemm_bf16_int4_ragged(const Tensor& a, const Tensor& b_q, cons
 Tensor op_moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_sf, const Tensor& w1_gs, const Tensor& w1_alpha,
                      const Tensor& w2_q, const Tensor& w2_sf, const Tensor& w2_gs, const Tensor& w2_alpha,
                      const Tensor& masked_m, const Tensor& in_gs, const Tensor& a2_gs) {
-  return moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m, in_gs, a2_gs, std::nullopt,
-                    std::nullopt, true);
+  const OptTensor out = moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m, in_gs, a2_gs,
+                                   std::nullopt, std::nullopt, true);
+  if (out) return *out;
+  Tensor r = moe_masked_steps({hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m, in_gs, a2_gs});
+  zero_dead_rows(r, masked_m);
+  return r;
 }
 
 TORCH_LIBRARY(mosaicist_sm100a, m) {

@@ -51,12 +51,24 @@ def moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alph
     layer takes 37.0 us fused against 40.0 us as separate kernels).  folded_alphas = fold_alphas(...)
     saves the GEMMs the division that folds the global scales into their alphas.
 
-    With the default configurations the layer is one native call (msc_moe_masked)."""
+    With the default configurations the layer is one native call (msc_moe_masked) for bf16 activations
+    and per-expert fp32 scales and alphas; whatever else the steps below take goes through them."""
     if (fuse_gemm1 is None or fuse_gemm1 == (w1_q.shape[1] % 256 == 0)) and masked_m is not None and \
             gemm1_config == _DEFAULT_CONFIG and gemm2_config == _DEFAULT_CONFIG:
         g1_alpha, g2_alpha = folded_alphas if folded_alphas is not None else (None, None)
-        return _host_ops.moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
-                                    input_global_scale, a2_global_scale, g1_alpha, g2_alpha)
+        if folded_alphas is None or (g1_alpha is not None and g2_alpha is not None):
+            out = _host_ops.moe_masked(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
+                                       input_global_scale, a2_global_scale, g1_alpha, g2_alpha)
+            if out is not None:
+                return out
+    return moe_masked_steps(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
+                            input_global_scale, a2_global_scale, gemm1_config, gemm2_config, fuse_gemm1, folded_alphas)
+
+
+def moe_masked_steps(hidden, w1_q, w1_sf, w1_gs, w1_alpha, w2_q, w2_sf, w2_gs, w2_alpha, masked_m,
+                     input_global_scale, a2_global_scale, gemm1_config=_DEFAULT_CONFIG,
+                     gemm2_config=_DEFAULT_CONFIG, fuse_gemm1: bool | None = None, folded_alphas=None):
+    """moe_masked as separate operators: quantise, fold the scales, GEMM1, activate + quantise, GEMM2."""
     a_q, a_sf = ops.quantize_nvfp4(hidden, input_global_scale, masked_m)
     g1_alpha, g2_alpha = folded_alphas if folded_alphas is not None else fold_alphas(
         w1_gs, w1_alpha, w2_gs, w2_alpha, input_global_scale, a2_global_scale)

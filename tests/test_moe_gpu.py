@@ -207,6 +207,54 @@ def test_moe_masked_matches_reference_layer(l, m, k, n):
     assert torch.equal(op, torch.where(rows_t, moe_masked(*args), torch.zeros_like(got)))
 
 
+@pytest.mark.parametrize("form", ["f32", "scalar", "strided", "folded_only", "wide_w2", "no_alpha"])
+@pytest.mark.parametrize("n", [256, 192])
+def test_moe_masked_takes_every_form_its_steps_take(form, n):
+    """The one-call layer reads bf16 activations and per-expert fp32 factors; fp32 activations, factors
+    to broadcast or copy, folded factors alone and a second weight of another width take the separate
+    steps, through the function and the torch operator alike."""
+    import mosaicist_b200.torch_ops  # noqa: F401
+    from mosaicist_b200 import _lib
+    from mosaicist_b200.moe import fold_alphas, moe_masked
+
+    l, m, k = 2, 128, 256
+    d = _dev_weights(_weights(l, k, n, seed=n))
+    rows = torch.tensor([128, 37], dtype=torch.int32, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    hidden = torch.randn((l, m, k), device="cuda", generator=gen).bfloat16()
+    gs, a2 = torch.full((l,), 500.0, device="cuda"), torch.full((l,), 800.0, device="cuda")
+    if form == "scalar":
+        d["w1_alpha"], d["w2_gs"] = torch.full((l,), 0.75, device="cuda"), torch.full((l,), 300.0, device="cuda")
+    w = [d[x] for x in ("w1_q", "w1_sf", "w1_gs", "w1_alpha", "w2_q", "w2_sf", "w2_gs", "w2_alpha")]
+    live = torch.arange(m, device="cuda")[None, :, None] < rows[:, None, None]
+    want = torch.where(live, moe_masked(hidden, *w, rows, gs, a2), 0)
+    assert int((want != 0).sum()) > 0.9 * int(live.sum()) * k
+    folded, operator = None, True
+    if form == "f32":
+        hidden = hidden.float()
+    elif form == "scalar":
+        w[3], w[6] = torch.tensor(0.75, device="cuda"), torch.tensor([300.0], device="cuda")
+    elif form == "strided":
+        w[2], w[7] = (torch.stack([x, torch.zeros_like(x)], 1)[:, 0] for x in (w[2], w[7]))
+        assert not w[2].is_contiguous()
+    elif form == "folded_only":
+        folded, operator = fold_alphas(w[2], w[3], w[6], w[7], gs, a2), False
+        w[2] = w[3] = w[6] = w[7] = None
+    elif form == "wide_w2":
+        w[4], w[5] = torch.cat([w[4], w[4]], 1).contiguous(), torch.cat([w[5], w[5]], 1).contiguous()
+        want = torch.cat([want, want], 2)
+    elif form == "no_alpha":            # a folded pair without the second factor: it counts as one
+        first, second = fold_alphas(w[2], w[3], w[6], w[7], gs, a2)
+        w[7] = torch.ones(l, device="cuda") * (a2 * w[6])
+        want = torch.where(live, moe_masked(hidden, *w, rows, gs, a2, folded_alphas=(first, torch.ones_like(second))), 0)
+        folded, operator = (first, None), False
+    got = moe_masked(hidden, *w, rows, gs, a2, folded_alphas=folded)
+    assert torch.equal(torch.where(live, got, 0), want)
+    if operator:
+        assert torch.equal(torch.ops.mosaicist_sm100a.moe_masked(hidden, *w, rows, gs, a2), want)
+    assert _lib.status_word() == 0
+
+
 @pytest.mark.parametrize("T_,E,k,h,n,first,local", [(256, 32, 4, 256, 128, 0, 32),
                                                      (384, 32, 2, 512, 256, 8, 8)])
 def test_megamoe_layer(T_, E, k, h, n, first, local):
