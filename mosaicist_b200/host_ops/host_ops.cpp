@@ -181,6 +181,12 @@ void need(const Tensor& t, const char* name, Types types, std::initializer_list<
     value_error(std::string(name) + " has shape " + shape_text(t.sizes()) + ", expected " +
                 shape_text(at::IntArrayRef(shape.begin(), shape.size())));
 }
+// A buffer of the caller's that a kernel reads or writes `elements` of, whatever shape it has.
+void need_room(const Tensor& t, const char* name, Types types, int64_t elements) {
+  need(t, name, types);
+  if (C10_UNLIKELY(t.numel() < elements))
+    value_error(std::string(name) + " holds " + std::to_string(t.numel()) + " elements, the call needs " + std::to_string(elements));
+}
 void need_dim(const Tensor& t, const char* name, int64_t dim) {
   if (C10_UNLIKELY(t.dim() != dim))
     value_error(std::string(name) + " must have " + std::to_string(dim) + " dimensions, got shape " + shape_text(t.sizes()));
@@ -361,6 +367,9 @@ std::tuple<Tensor, Tensor> quantize_mxfp8(const Tensor& x, bool tiled, const Opt
   if (fresh) {
     q = empty({total, k}, at::kByte, x);
     sf = tiled ? empty({(total + 127) / 128, k / 128, 32, 16}, at::kByte, x) : empty({total, k / 32}, at::kByte, x);
+  } else {
+    need_room(*q, "q", kBytes, total * k);
+    need_room(*sf, "sf", kBytes, tiled ? (total + 127) / 128 * (k / 128) * 512 : total * (k / 32));
   }
   const Lib& f = lib();
   void* st = stream();
@@ -382,8 +391,8 @@ Tensor gemm_f16(const Tensor& a, const Tensor& b, OptTensor out, int max_ctas) {
     value_error("a and b must be CUDA tensors with unit stride along their rows");
   const int64_t m = a.size(0), k = a.size(1), n = b.size(1);
   if (!out) out = empty({m, n}, t, a);
-  else if (out->scalar_type() != t || out->dim() != 2 || out->size(0) != m || out->size(1) != n || out->stride(1) != 1)
-    value_error("out must be (m, n) in the input dtype with unit stride along rows");
+  else if (!out->is_cuda() || out->scalar_type() != t || out->dim() != 2 || out->size(0) != m || out->size(1) != n || out->stride(1) != 1)
+    value_error("out must be an (m, n) CUDA tensor in the input dtype with unit stride along rows");
   const Lib& f = lib();
   void* st = stream();
   launch([&] {
@@ -400,6 +409,7 @@ Tensor dequant_int4(const Tensor& b_q, const Tensor& scales, int64_t group_size,
   if (group_size <= 0) value_error("group_size must be positive");
   need(scales, "scales", kBf16, {l, n, k / group_size});
   if (!out) out = empty({l, n, k}, at::kBFloat16, b_q);
+  else need_room(*out, "out", kBf16, l * n * k);
   const Lib& f = lib();
   void* st = stream();
   launch([&] { return f.msc_int4_dequant_bf16(ptr(b_q), ptr(scales), out->data_ptr(), l, n, k, group_size, st); });
@@ -417,6 +427,7 @@ Tensor gemm_bf16_ragged(const Tensor& a, const Tensor& b, const Tensor& offsets,
   need(rows, "group_rows", kI32, {l});
   if (alpha) need(*alpha, "alpha", kF32, {l});
   if (!out) out = empty({total, n}, at::kBFloat16, a);
+  else need_room(*out, "out", kBf16, total * n);
   const Lib& f = lib();
   void* st = stream();
   launch([&] {
@@ -450,6 +461,7 @@ Tensor gemm_int4_ragged(const Tensor& a, const Tensor& b_q, const Tensor& scales
   need(rows, "group_rows", kI32, {l});
   if (alpha) need(*alpha, "alpha", kF32, {l});
   if (!out) out = empty({total, n}, at::kBFloat16, a);
+  else need_room(*out, "out", kBf16, total * n);
   const Lib& f = lib();
   void* st = stream();
   launch([&] {
@@ -692,6 +704,9 @@ void route(const Layer& layer, const Tensor& logits) {
   ATTR(ids); ATTR(weights); ATTR(topk);
   need_dim(logits, "logits", 2);
   const int64_t tokens = logits.size(0), experts = logits.size(1), topk = layer.num(s_topk);
+  need_room(logits, "logits", kF32, tokens * experts);
+  need_room(layer.t(s_ids), "ids", kI32, tokens * topk);
+  need_room(layer.t(s_weights), "weights", kF32, tokens * topk);
   int32_t* ids = layer.p<int32_t>(s_ids);
   float* weights = layer.p<float>(s_weights);
   const Lib& f = lib();
@@ -712,9 +727,13 @@ PY_FUNCTION(moe_dispatch, 3) {
   ATTR(rows_cap);
   const Layer layer{a[0]};
   const Tensor& tokens = tensor(a[1], "tokens");
-  if (a[2] != Py_None) route(layer, tensor(a[2], "logits"));
+  if (tokens.dim() < 1) value_error("tokens must have a dimension of tokens");
   const int64_t T = tokens.size(0), K = layer.num(s_topk), E = layer.num(s_E), first = layer.num(s_expert_first);
   const int64_t h = layer.num(s_h), cap = layer.num(s_rows_cap);
+  need(tokens, "tokens", kBf16);
+  if (tokens.numel() != T * h) value_error("tokens has shape " + shape_text(tokens.sizes()) + ", expected " + shape_text({T, h}));
+  for (PyObject* name : {s_ids, s_rank}) need_room(layer.t(name), "ids / rank", kI32, T * K);
+  if (a[2] != Py_None) route(layer, tensor(a[2], "logits"));
   int32_t *ids = layer.p<int32_t>(s_ids), *rank = layer.p<int32_t>(s_rank), *rows = layer.p<int32_t>(s_group_rows);
   int32_t *offsets = layer.p<int32_t>(s_group_offsets), *total = layer.p<int32_t>(s_total_rows), *scratch = layer.p<int32_t>(s_scratch);
   PyObject* staged = layer.get(s_sf_rows);
@@ -741,6 +760,7 @@ PY_FUNCTION(moe_combine, 3) {
   const int64_t T = tokens.size(0), h = layer.num(s_h);
   OptTensor out = opt_tensor(a[2], "out");
   if (!out) out = empty({T, h}, at::kBFloat16, tokens);
+  else need_room(*out, "out", kBf16, T * h);
   const int64_t K = layer.num(s_topk), first = layer.num(s_expert_first), E = layer.num(s_E);
   const void* y = layer.p<void>(s_y);
   const int32_t *ids = layer.p<int32_t>(s_ids), *rank = layer.p<int32_t>(s_rank), *offsets = layer.p<int32_t>(s_group_offsets);
