@@ -22,9 +22,11 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
+#include <deque>
 #include <initializer_list>
 #include <optional>
 #include <tuple>
+#include <vector>
 
 #include "../../include/mosaicist_sm100a.h"
 
@@ -687,20 +689,42 @@ PY_FUNCTION(moe_masked, 14) {
 
 struct Layer {
   PyObject* self;
+  std::deque<Tensor> held;    // what the call uses stays alive until it returns, whoever rebinds the attribute
+  int64_t num(PyObject* name) {
+    PyObject* v = get(name);
+    const long long n = PyLong_AsLongLong(v);
+    Py_DECREF(v);
+    if (n == -1 && PyErr_Occurred()) raise();
+    return n;
+  }
+  // null where the attribute is None
+  const Tensor* opt(PyObject* name) {
+    PyObject* v = get(name);
+    const bool none = v == Py_None, tensor = !none && THPVariable_Check(v);
+    if (tensor) held.push_back(THPVariable_Unpack(v));
+    Py_DECREF(v);
+    if (none) return nullptr;
+    if (!tensor) value_error("a buffer of the layer is not a tensor");
+    return &held.back();
+  }
+  const Tensor& t(PyObject* name) {
+    const Tensor* v = opt(name);
+    if (!v) value_error("a buffer of the layer is missing");
+    return *v;
+  }
+  template <class T>
+  T* p(PyObject* name) { return static_cast<T*>(t(name).data_ptr()); }
+
+ private:
   PyObject* get(PyObject* name) const {
     PyObject* v = PyObject_GetAttr(self, name);
     if (!v) raise();
-    Py_DECREF(v);   // the layer keeps it alive during the call
     return v;
   }
-  int64_t num(PyObject* name) const { return integer(get(name)); }
-  const Tensor& t(PyObject* name) const { return tensor(get(name), "layer buffer"); }
-  template <class T>
-  T* p(PyObject* name) const { return static_cast<T*>(t(name).data_ptr()); }
 };
 #define ATTR(name) static PyObject* const s_##name = PyUnicode_InternFromString(#name)
 
-void route(const Layer& layer, const Tensor& logits) {
+void route(Layer& layer, const Tensor& logits) {
   ATTR(ids); ATTR(weights); ATTR(topk);
   need_dim(logits, "logits", 2);
   const int64_t tokens = logits.size(0), experts = logits.size(1), topk = layer.num(s_topk);
@@ -716,7 +740,8 @@ void route(const Layer& layer, const Tensor& logits) {
 
 // route(self, logits)
 PY_FUNCTION(moe_route, 2) {
-  route(Layer{a[0]}, tensor(a[1], "logits"));
+  Layer layer{a[0]};
+  route(layer, tensor(a[1], "logits"));
   Py_RETURN_NONE;
 }
 
@@ -725,7 +750,7 @@ PY_FUNCTION(moe_dispatch, 3) {
   ATTR(ids); ATTR(weights); ATTR(rank); ATTR(group_rows); ATTR(group_offsets); ATTR(total_rows); ATTR(scratch); ATTR(topk);
   ATTR(E); ATTR(expert_first); ATTR(input_gs); ATTR(h); ATTR(a_q); ATTR(a_sf); ATTR(row_weight); ATTR(row_token); ATTR(sf_rows);
   ATTR(rows_cap);
-  const Layer layer{a[0]};
+  Layer layer{a[0]};
   const Tensor& tokens = tensor(a[1], "tokens");
   if (tokens.dim() < 1) value_error("tokens must have a dimension of tokens");
   const int64_t T = tokens.size(0), K = layer.num(s_topk), E = layer.num(s_E), first = layer.num(s_expert_first);
@@ -736,8 +761,8 @@ PY_FUNCTION(moe_dispatch, 3) {
   if (a[2] != Py_None) route(layer, tensor(a[2], "logits"));
   int32_t *ids = layer.p<int32_t>(s_ids), *rank = layer.p<int32_t>(s_rank), *rows = layer.p<int32_t>(s_group_rows);
   int32_t *offsets = layer.p<int32_t>(s_group_offsets), *total = layer.p<int32_t>(s_total_rows), *scratch = layer.p<int32_t>(s_scratch);
-  PyObject* staged = layer.get(s_sf_rows);
-  void* sf_rows = staged == Py_None ? nullptr : tensor(staged, "sf_rows").data_ptr();
+  const Tensor* staged = layer.opt(s_sf_rows);
+  void* sf_rows = staged ? staged->data_ptr() : nullptr;
   const float *weights = layer.p<float>(s_weights), *gs = layer.p<float>(s_input_gs);
   void *a_q = layer.p<void>(s_a_q), *a_sf = layer.p<void>(s_a_sf);
   float* row_weight = layer.p<float>(s_row_weight);
@@ -755,7 +780,7 @@ PY_FUNCTION(moe_dispatch, 3) {
 // combine(self, tokens, out or None) -> out: the sum of each token's expert rows
 PY_FUNCTION(moe_combine, 3) {
   ATTR(y); ATTR(ids); ATTR(rank); ATTR(group_offsets); ATTR(h); ATTR(topk); ATTR(expert_first); ATTR(E);
-  const Layer layer{a[0]};
+  Layer layer{a[0]};
   const Tensor& tokens = tensor(a[1], "tokens");
   const int64_t T = tokens.size(0), h = layer.num(s_h);
   OptTensor out = opt_tensor(a[2], "out");

@@ -76,3 +76,31 @@ def test_routed_layer_buffers():
              _t(T, E, dtype=F32, device="cpu"))
     _refused(lambda b: _host_ops.moe_route(layer, b), _t(T + 1, E, dtype=F32), _t(T, E))
     _refused(lambda b: _host_ops.moe_combine(layer, tokens, b), *_bad(T, h, BF16, F32))
+
+
+def test_layer_attributes_may_be_computed():
+    """A buffer that only the attribute look-up itself holds stays alive for the call."""
+    from mosaicist_b200.moe import _host_ops
+
+    asked = []
+
+    class Layer:
+        topk = 2
+
+        @property
+        def ids(self):
+            asked.append("ids")
+            return _t(16, 2, dtype=I32)
+
+        @property
+        def weights(self):
+            asked.append("weights")
+            return _t(15, 2, dtype=F32)
+
+    for _ in range(20):
+        with pytest.raises(ValueError, match="weights holds 30 elements"):
+            _host_ops.moe_route(Layer(), _t(16, 8, dtype=F32))
+    assert asked[:2] == ["ids", "weights"]
+    Layer.ids = None
+    with pytest.raises(ValueError, match="missing"):
+        _host_ops.moe_route(Layer(), _t(16, 8, dtype=F32))
