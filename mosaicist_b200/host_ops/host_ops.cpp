@@ -22,8 +22,10 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
+#include <atomic>
 #include <deque>
 #include <initializer_list>
+#include <memory>
 #include <optional>
 #include <tuple>
 #include <vector>
@@ -49,9 +51,9 @@ struct Lib {
 #define X(name) decltype(&::name) name = nullptr;
   MSC_ENTRY_POINTS(X)
 #undef X
-  bool bound = false;
 };
-Lib g_lib;
+// Set once, when it is complete: a thread without the GIL sees all of the table or none of it.
+std::atomic<const Lib*> g_lib{nullptr};
 
 struct Gil {
   PyGILState_STATE s = PyGILState_Ensure();
@@ -65,20 +67,22 @@ struct Gil {
   throw e;
 }
 
-// Fetches the addresses on first use: mosaicist_b200._lib.addresses() loads the library.
-void bind() {
+// Fetches the addresses on first use: mosaicist_b200._lib.addresses() loads the library.  Threads that
+// meet here each fetch them (the GIL may change hands during the import, so nobody waits for another
+// thread while holding it); the first table stays.
+const Lib* bind() {
   Gil gil;
   PyObject* mod = PyImport_ImportModule("mosaicist_b200._lib");
   if (!mod) raise();
   PyObject* table = PyObject_CallMethod(mod, "addresses", nullptr);
   Py_DECREF(mod);
   if (!table) raise();
-  Lib lib;
+  auto lib = std::make_unique<Lib>();
 #define X(name)                                                                        \
   {                                                                                    \
     PyObject* a = PyDict_GetItemString(table, #name);                                  \
-    lib.name = a ? reinterpret_cast<decltype(&::name)>(PyLong_AsVoidPtr(a)) : nullptr; \
-    if (!lib.name) {                                                                   \
+    lib->name = a ? reinterpret_cast<decltype(&::name)>(PyLong_AsVoidPtr(a)) : nullptr; \
+    if (!lib->name) {                                                                  \
       Py_DECREF(table);                                                                \
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "no address for " #name); \
       raise();                                                            \
@@ -87,13 +91,14 @@ void bind() {
   MSC_ENTRY_POINTS(X)
 #undef X
   Py_DECREF(table);
-  lib.bound = true;
-  g_lib = lib;
+  const Lib* seen = nullptr;
+  if (!g_lib.compare_exchange_strong(seen, lib.get(), std::memory_order_acq_rel, std::memory_order_acquire)) return seen;
+  return lib.release();
 }
 
 const Lib& lib() {
-  if (C10_UNLIKELY(!g_lib.bound)) bind();
-  return g_lib;
+  const Lib* l = g_lib.load(std::memory_order_acquire);
+  return C10_LIKELY(l != nullptr) ? *l : *bind();
 }
 
 // Raises mosaicist_b200._lib.MscError for a status other than MSC_OK.
@@ -102,7 +107,7 @@ void check(int code) {
   Gil gil;
   PyObject* mod = PyImport_ImportModule("mosaicist_b200._lib");
   if (mod) {
-    const char* text = g_lib.msc_last_error();
+    const char* text = lib().msc_last_error();
     PyObject* type = PyObject_GetAttrString(mod, "MscError");
     PyObject* exc = type ? PyObject_CallFunction(type, "is", code, text && *text ? text : "libmosaicist_sm100a call failed") : nullptr;
     if (exc) PyErr_SetObject(type, exc);

@@ -104,3 +104,42 @@ def test_layer_attributes_may_be_computed():
     Layer.ids = None
     with pytest.raises(ValueError, match="missing"):
         _host_ops.moe_route(Layer(), _t(16, 8, dtype=F32))
+
+
+def test_first_calls_from_several_threads():
+    """The library's entry points are fetched by whichever threads call first: all of them get a whole
+    table and none waits for another.  (In a process of its own: the table is fetched once.)"""
+    import pathlib
+    import subprocess
+    import sys
+
+    code = """
+import threading, time, torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from mosaicist_b200 import _lib, ops
+fetch, calls = _lib.addresses, []
+def slow():
+    calls.append(1)
+    time.sleep(0.2)                  # other threads get the GIL here
+    return fetch()
+_lib.addresses = slow
+with FakeTensorMode():
+    a, b = (torch.empty(s, dtype=torch.bfloat16, device="cuda") for s in ((64, 128), (128, 64)))
+    out = torch.empty((64, 64), dtype=torch.bfloat16, device="cuda")
+seen = []
+def call():
+    try:
+        ops.gemm_f16(a, b, out=out)  # no memory behind the tensors: refused by torch or the library
+    except RuntimeError as e:
+        seen.append(str(e))
+threads = [threading.Thread(target=call) for _ in range(8)]
+[t.start() for t in threads]
+[t.join(60) for t in threads]
+assert len(seen) == 8 and not any(t.is_alive() for t in threads), seen
+assert not any("no address" in s for s in seen), seen
+n = len(calls)
+call()
+assert 1 <= n <= 8 and len(calls) == n and len(seen) == 9
+"""
+    root = pathlib.Path(__file__).resolve().parents[1]
+    subprocess.run([sys.executable, "-W", "ignore", "-c", code], check=True, cwd=root, timeout=240)
