@@ -61,6 +61,11 @@ typedef struct msc_gemm_cfg {
 } msc_gemm_cfg;
 
 int msc_version(void);
+
+/* Digest of the declarations in this header that the library was built from (empty if the build did
+ * not pass one).  A binding with fixed signatures compares it with its own. */
+const char* msc_abi(void);
+
 const char* msc_last_error(void);
 
 /* Releases what the library caches on the host: the encoded tensor maps, keyed by (address,

@@ -36,6 +36,7 @@ _CFG = ctypes.POINTER(GemmCfg)
 #: every symbol include/mosaicist_sm100a.h declares: name -> (restype, argtypes)
 SIGNATURES = {
     "msc_version": (_I, []),
+    "msc_abi": (ctypes.c_char_p, []),
     "msc_last_error": (ctypes.c_char_p, []),
     "msc_shutdown": (_I, []),
     "msc_ptx_path": (ctypes.c_char_p, []),
@@ -97,15 +98,26 @@ def load() -> ctypes.CDLL:
 
 
 def host_ops():
-    """The native host path (host_ops/host_ops.cpp), built on first use where it is missing."""
-    try:
-        from . import _host_ops
-    except ImportError:
-        from . import build
+    """The native host path (host_ops/host_ops.cpp), built first where it is missing or was built from
+    another source or for another torch."""
+    from . import build
 
-        build.build_host_ops(force=True)
-        from . import _host_ops
+    build.build_host_ops()
+    from . import _host_ops
     return _host_ops
+
+
+class _HostOps:
+    """host_ops(), loaded when the first of its functions is asked for: importing this package needs
+    neither a compiler nor the built module."""
+
+    def __getattr__(self, name):
+        mod = host_ops()
+        self.__dict__.update({n: getattr(mod, n) for n in dir(mod) if not n.startswith("_")})
+        return getattr(mod, name)
+
+
+native = _HostOps()
 
 
 def addresses() -> dict:

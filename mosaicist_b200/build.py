@@ -12,7 +12,12 @@ runs on a CPU-only machine; the resulting .so is what the GPU machine loads.
 
 from __future__ import annotations
 
+import contextlib
+import fcntl
+import hashlib
+import os
 import pathlib
+import re
 import shutil
 import subprocess
 import sys
@@ -20,6 +25,7 @@ import sys
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libmosaicist_sm100a.so"
+HEADER = PKG.parent / "include" / "mosaicist_sm100a.h"
 PTXAS_LOG = PKG / "libmosaicist_sm100a.ptxas.log"
 DEBUG_LIB = PKG / "libmosaicist_sm100a_debug.so"
 
@@ -35,7 +41,7 @@ def _stale() -> bool:
     if not LIB.exists():
         return True
     built = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*")) + [PKG.parent / "include" / "mosaicist_sm100a.h"]
+    deps = list(CSRC.glob("*")) + [HEADER]
     return any(p.stat().st_mtime > built for p in deps)
 
 
@@ -51,7 +57,7 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
             return LIB  # prebuilt library on a machine without the toolkit
         raise RuntimeError("nvcc not found and no prebuilt libmosaicist_sm100a.so")
     srcs = [str(s) for s in sources()]
-    cmd = [nvcc, *ARCH, *COMMON, "-Xptxas", "-v", "-t", "0", "-shared", "-Xcompiler", "-fPIC",
+    cmd = [nvcc, *ARCH, *COMMON, f'-DMSC_ABI="{abi()}"', "-Xptxas", "-v", "-t", "0", "-shared", "-Xcompiler", "-fPIC",
            "-cudart", "static", "-o", str(LIB), *srcs, "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     PTXAS_LOG.write_text(res.stderr)
@@ -64,20 +70,53 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
 
 HOST_OPS_SRC = PKG / "host_ops" / "host_ops.cpp"
 HOST_OPS = PKG / "_host_ops.so"
+HOST_OPS_STAMP = PKG / "_host_ops.stamp"
+
+
+def abi() -> str:
+    """Digest of what the header declares, comments left out: the library and the host path were built
+    for each other if theirs are equal."""
+    text = re.sub(r"/\*.*?\*/|//[^\n]*", " ", HEADER.read_text(), flags=re.S)
+    return hashlib.sha256(" ".join(text.split()).encode()).hexdigest()[:16]
+
+
+def host_ops_stamp() -> str:
+    """What an existing host path must have been built from: its source, the header, and the torch and
+    Python whose C++ interfaces it is tied to."""
+    import torch
+
+    source = hashlib.sha256(HOST_OPS_SRC.read_bytes()).hexdigest()[:16]
+    return f"source {source} header {abi()} torch {torch.__version__} python {sys.version_info[:2]} {sys.platform}"
+
+
+def host_ops_current() -> bool:
+    try:
+        return HOST_OPS.exists() and HOST_OPS_STAMP.read_text() == host_ops_stamp()
+    except OSError:
+        return False
+
+
+@contextlib.contextmanager
+def _locked(path: pathlib.Path):
+    """One process at a time; the others wait."""
+    with open(path, "a") as f:
+        fcntl.flock(f, fcntl.LOCK_EX)
+        try:
+            yield
+        finally:
+            fcntl.flock(f, fcntl.LOCK_UN)
 
 
 def build_host_ops(force: bool = False) -> pathlib.Path:
     """The native host path of the operators (host_ops/host_ops.cpp), a Python extension module
-    against torch's C++ interface; returns its path."""
-    deps = [HOST_OPS_SRC, PKG.parent / "include" / "mosaicist_sm100a.h"]
-    if not force and HOST_OPS.exists() and all(p.stat().st_mtime <= HOST_OPS.stat().st_mtime for p in deps):
+    against torch's C++ interface; returns its path.  Ranks that start together build it once: they
+    take turns, and the module appears in place when it is complete."""
+    if not force and host_ops_current():
         return HOST_OPS
     gxx = shutil.which("g++")
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if gxx is None:
-        if HOST_OPS.exists():
-            return HOST_OPS  # prebuilt module on a machine without a compiler
-        raise RuntimeError("g++ not found and no prebuilt _host_ops.so")
+        raise RuntimeError("g++ not found and no _host_ops.so that fits this source, torch and Python")
     import sysconfig
 
     import torch
@@ -86,13 +125,24 @@ def build_host_ops(force: bool = False) -> pathlib.Path:
     cuda = pathlib.Path(nvcc).resolve().parents[1]
     includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
                 sysconfig.get_paths()["include"]]
-    cmd = [gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in includes],
-           "-o", str(HOST_OPS), str(HOST_OPS_SRC), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
-           "-ltorch_cuda", "-lc10", "-lc10_cuda"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("g++ failed on the host operators:\n" + res.stderr[-4000:])
+    with _locked(PKG / "_host_ops.lock"):
+        if not force and host_ops_current():
+            return HOST_OPS
+        stamp = host_ops_stamp()
+        part = PKG / f"_host_ops.{os.getpid()}.part"
+        cmd = [gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f'-DMSC_ABI="{abi()}"',
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in includes],
+               "-o", str(part), str(HOST_OPS_SRC), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+               "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+        try:
+            res = subprocess.run(cmd, capture_output=True, text=True)
+            if res.returncode != 0:
+                raise RuntimeError("g++ failed on the host operators:\n" + res.stderr[-4000:])
+            os.replace(part, HOST_OPS)
+            part.write_text(stamp)
+            os.replace(part, HOST_OPS_STAMP)
+        finally:
+            part.unlink(missing_ok=True)
     return HOST_OPS
 
 
@@ -122,11 +172,11 @@ def build_cupti_shim(force: bool = False) -> pathlib.Path | None:
 
 def build_debug(force: bool = False) -> pathlib.Path:
     """The -DMSC_DEBUG build (clock stamps, skip flags); returns its path."""
-    deps = list(CSRC.glob("*")) + [PKG.parent / "include" / "mosaicist_sm100a.h"]
+    deps = list(CSRC.glob("*")) + [HEADER]
     if not force and DEBUG_LIB.exists() and all(p.stat().st_mtime <= DEBUG_LIB.stat().st_mtime for p in deps):
         return DEBUG_LIB
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    cmd = [nvcc, *ARCH, *COMMON, "-DMSC_DEBUG", "-shared", "-Xcompiler", "-fPIC", "-cudart", "static",
+    cmd = [nvcc, *ARCH, *COMMON, f'-DMSC_ABI="{abi()}"', "-DMSC_DEBUG", "-shared", "-Xcompiler", "-fPIC", "-cudart", "static",
            "-o", str(DEBUG_LIB), *[str(s) for s in sources()], "-ldl"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

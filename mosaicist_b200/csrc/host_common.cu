@@ -205,6 +205,11 @@ extern "C" {
 
 int msc_version(void) { return 1; }
 
+#ifndef MSC_ABI
+#define MSC_ABI ""
+#endif
+const char* msc_abi(void) { return MSC_ABI; }
+
 int msc_shutdown(void) {
   msc::clear_tmap_cache();
   return MSC_OK;

@@ -8,7 +8,8 @@
 // Two fronts over the same functions on at::Tensor:
 //   - a CPython module (METH_FASTCALL, positional arguments only): mosaicist_b200.ops and
 //     mosaicist_b200.moe keep their documented signatures and pass everything on;
-//   - torch operators mosaicist_sm100a::* (mosaicist_b200.torch_ops adds the shape functions).
+//   - kernels of the torch operators mosaicist_sm100a::* (mosaicist_b200.torch_ops has their schemas
+//     and shape functions).
 // The library is not linked: its entry points come as addresses from mosaicist_b200._lib, which
 // decides which build is loaded and raises if there is none.
 #define PY_SSIZE_T_CLEAN
@@ -22,13 +23,14 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
+#include <string.h>
+
 #include <atomic>
 #include <deque>
 #include <initializer_list>
 #include <memory>
 #include <optional>
 #include <tuple>
-#include <vector>
 
 #include "../../include/mosaicist_sm100a.h"
 
@@ -40,7 +42,7 @@ using OptTensor = std::optional<Tensor>;
 // ---- the library's entry points ---------------------------------------------------------------
 
 #define MSC_ENTRY_POINTS(X)                                                                      \
-  X(msc_last_error) X(msc_grouped_gemm_nvfp4) X(msc_grouped_gemm_nvfp4_ragged)                   \
+  X(msc_abi) X(msc_last_error) X(msc_grouped_gemm_nvfp4) X(msc_grouped_gemm_nvfp4_ragged)                   \
   X(msc_grouped_gemm_nvfp4_swiglu_ragged) X(msc_grouped_gemm_mxfp8_ragged) X(msc_quantize_rows)  \
   X(msc_amax_global_scale) X(msc_gemm_f16) X(msc_int4_dequant_bf16)                              \
   X(msc_grouped_gemm_bf16_ragged) X(msc_grouped_gemm_bf16_int4_ragged) X(msc_moe_route_topk)     \
@@ -91,6 +93,14 @@ const Lib* bind() {
   MSC_ENTRY_POINTS(X)
 #undef X
   Py_DECREF(table);
+#ifdef MSC_ABI
+  const char* abi = lib->msc_abi();
+  if (abi && *abi && strcmp(abi, MSC_ABI) != 0) {
+    PyErr_SetString(PyExc_RuntimeError, "libmosaicist_sm100a and the host path were built from different headers: "
+                                        "run `python -m mosaicist_b200.build`");
+    raise();
+  }
+#endif
   const Lib* seen = nullptr;
   if (!g_lib.compare_exchange_strong(seen, lib.get(), std::memory_order_acq_rel, std::memory_order_acquire)) return seen;
   return lib.release();
@@ -882,24 +892,7 @@ Tensor op_moe_masked(const Tensor& hidden, const Tensor& w1_q, const Tensor& w1_
   return r;
 }
 
-TORCH_LIBRARY(mosaicist_sm100a, m) {
-  m.set_python_module("mosaicist_b200.torch_ops");   // where the shape functions are
-  const std::vector<at::Tag> tags = {at::Tag::pt2_compliant_tag};
-  m.def("grouped_gemm_nvfp4(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor? alpha, Tensor? masked_m) -> Tensor", tags);
-  m.def("grouped_gemm_nvfp4_ragged(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor group_offsets, Tensor group_rows, "
-        "Tensor? alpha, Tensor? row_scale) -> Tensor", tags);
-  m.def("quantize_nvfp4(Tensor x, Tensor global_scale, Tensor? masked_m) -> (Tensor, Tensor)", tags);
-  m.def("silu_mul_quantize_nvfp4(Tensor gateup, Tensor global_scale, Tensor? masked_m) -> (Tensor, Tensor)", tags);
-  m.def("global_scale_for(Tensor x) -> Tensor", tags);
-  m.def("quantize_mxfp8(Tensor x) -> (Tensor, Tensor)", tags);
-  m.def("grouped_gemm_mxfp8_ragged(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor group_offsets, Tensor group_rows, "
-        "Tensor? alpha, Tensor? row_scale) -> Tensor", tags);
-  m.def("gemm_f16(Tensor a, Tensor b) -> Tensor", tags);
-  m.def("grouped_gemm_bf16_int4_ragged(Tensor a, Tensor b_q, Tensor scales, Tensor group_offsets, Tensor group_rows, "
-        "Tensor? alpha, int group_size) -> Tensor", tags);
-  m.def("moe_masked(Tensor hidden, Tensor w1_q, Tensor w1_sf, Tensor w1_gs, Tensor w1_alpha, Tensor w2_q, Tensor w2_sf, "
-        "Tensor w2_gs, Tensor w2_alpha, Tensor masked_m, Tensor input_global_scale, Tensor a2_global_scale) -> Tensor", tags);
-}
+// The operators' schemas are in mosaicist_b200.torch_ops.
 TORCH_LIBRARY_IMPL(mosaicist_sm100a, CUDA, m) {
   m.impl("grouped_gemm_nvfp4", op_grouped_gemm_nvfp4);
   m.impl("grouped_gemm_nvfp4_ragged", op_grouped_gemm_nvfp4_ragged);

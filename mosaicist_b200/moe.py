@@ -18,7 +18,7 @@ import torch
 
 from . import _lib, ops
 
-_host_ops = _lib.host_ops()
+_host_ops = _lib.native
 
 
 _OFFSETS = {}

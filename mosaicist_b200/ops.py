@@ -13,7 +13,7 @@ import torch
 
 from . import _lib
 
-_host_ops = _lib.host_ops()
+_host_ops = _lib.native
 
 
 @dataclass(frozen=True)

@@ -16,19 +16,44 @@ that build graphs of torch operators (tracing, FakeTensor shape propagation) ins
     moe_masked                 the masked MoE layer, arguments of the reference's moe_masked
                                (experiments/flashinfer-megamoe-sm100a/moe.py:47-79)
 
-Each is the corresponding C-ABI entry point, defined natively (host_ops/host_ops.cpp) so that a
-call costs the dispatcher and the launch; this module adds the shape functions.  Operators return
-fresh tensors, so rows a masked call leaves untouched come back as zeros.  Importing this module
-registers the operators; it needs no GPU.
+Each is the corresponding C-ABI entry point; their kernels are native (host_ops/host_ops.cpp), so that
+a call costs the dispatcher and the launch.  Here are their schemas and shape functions: operators
+can be traced without a GPU, and without the native module where that cannot be built.  Operators
+return fresh tensors, so rows a masked call leaves untouched come back as zeros.  None has a derivative.
 """
 
 from __future__ import annotations
+
+import warnings
 
 import torch
 
 from . import _lib
 
-_lib.host_ops()     # defines the operators
+if "_LIBRARY" in globals():     # the module is being reloaded
+    _LIBRARY._destroy()
+_LIBRARY = torch.library.Library("mosaicist_sm100a", "DEF")
+for _schema in (
+        "grouped_gemm_nvfp4(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor? alpha, Tensor? masked_m) -> Tensor",
+        "grouped_gemm_nvfp4_ragged(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor group_offsets, "
+        "Tensor group_rows, Tensor? alpha, Tensor? row_scale) -> Tensor",
+        "quantize_nvfp4(Tensor x, Tensor global_scale, Tensor? masked_m) -> (Tensor, Tensor)",
+        "silu_mul_quantize_nvfp4(Tensor gateup, Tensor global_scale, Tensor? masked_m) -> (Tensor, Tensor)",
+        "global_scale_for(Tensor x) -> Tensor",
+        "quantize_mxfp8(Tensor x) -> (Tensor, Tensor)",
+        "grouped_gemm_mxfp8_ragged(Tensor a_q, Tensor a_sf, Tensor b_q, Tensor b_sf, Tensor group_offsets, "
+        "Tensor group_rows, Tensor? alpha, Tensor? row_scale) -> Tensor",
+        "gemm_f16(Tensor a, Tensor b) -> Tensor",
+        "grouped_gemm_bf16_int4_ragged(Tensor a, Tensor b_q, Tensor scales, Tensor group_offsets, Tensor group_rows, "
+        "Tensor? alpha, int group_size) -> Tensor",
+        "moe_masked(Tensor hidden, Tensor w1_q, Tensor w1_sf, Tensor w1_gs, Tensor w1_alpha, Tensor w2_q, Tensor w2_sf, "
+        "Tensor w2_gs, Tensor w2_alpha, Tensor masked_m, Tensor input_global_scale, Tensor a2_global_scale) -> Tensor"):
+    _LIBRARY.define(_schema, tags=(torch.Tag.pt2_compliant_tag,))
+
+try:
+    _lib.host_ops()     # registers the kernels
+except (ImportError, OSError, RuntimeError) as _why:
+    warnings.warn(f"the operators mosaicist_sm100a::* can be traced but not run: {_why}")
 _OPS = torch.ops.mosaicist_sm100a
 grouped_gemm_nvfp4 = _OPS.grouped_gemm_nvfp4
 grouped_gemm_nvfp4_ragged = _OPS.grouped_gemm_nvfp4_ragged
@@ -43,7 +68,7 @@ moe_masked = _OPS.moe_masked
 
 
 def _fake(name):
-    return torch.library.register_fake(f"mosaicist_sm100a::{name}")
+    return torch.library.register_fake(f"mosaicist_sm100a::{name}", lib=_LIBRARY)
 
 
 @_fake("grouped_gemm_nvfp4")
