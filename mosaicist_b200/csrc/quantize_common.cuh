@@ -38,10 +38,15 @@ __device__ __forceinline__ float silu_mul(float gate, float up) {
   return __fmul_rn(__fmul_rn(s, gate), up);
 }
 
-// a / b rounded to nearest, given rb = RN(1 / b): one multiply and two fused multiply-adds
-// (q = RN(a rb); r = a - q b exactly; q' = RN(q + r rb)), which is the correctly rounded
-// quotient whenever rb is the correctly rounded reciprocal and nothing overflows; the block
-// quantiser divides 16 values by the same step, so the reciprocal is shared.
+// a / b by one correction step: q = RN(a rb), r = RN(a - q b), q' = RN(q + r rb).  The method is
+// Markstein's (P. W. Markstein, Computation of elementary functions on the IBM RISC System/6000
+// processor, IBM J. Res. Dev. 34(1), 1990): with rb = RN(1 / b), q within one ulp of a / b, and r exact,
+// q' is a / b correctly rounded.  r is exact while nothing over- or underflows (q finite, q * b and r
+// within fp32's exponents).  q may miss by more than one ulp where a's significand is the smaller one,
+// so what this file relies on is tested on the device over all significands against __fdiv_rn
+// (tests/test_division_gpu.py): the quotients that become scales, bit for bit, and the e2m1 values of
+// quotients around every rounding boundary.  The block quantiser divides 16 values by the same step,
+// so the reciprocal is shared.
 template <bool GUARD = true>
 __device__ __forceinline__ float div_rn_shared_rcp(float a, float b, float rb) {
   const float q = __fmul_rn(a, rb);
@@ -102,11 +107,19 @@ __device__ __forceinline__ void pack_block(const float* v, float safe, float rsa
   }
 }
 
-// a / b rounded to nearest, through rb = RN(1 / b) where every intermediate of the shared-
-// reciprocal form is a normal number (a zero or between 1e-30 and 1e30), else by division.
+// a / b rounded to nearest, through rb = RN(1 / b) where every intermediate is in range for b = 6 (a
+// zero or between 1e-30 and 1e30: the remainder of 1e-30 is a multiple of 2^-147), else by division.
 __device__ __forceinline__ float div_rn_mid(float a, float b, float rb) {
   if (a == 0.0f || (a >= 1e-30f && a <= 1e30f)) return div_rn_shared_rcp<false>(a, b, rb);
   return __fdiv_rn(a, b);
+}
+// The block maximum's share of a scale, amax / 6, and the step that a scale stands for, sf / gs with sf
+// an e4m3 value (0 or 2^-9 .. 448): both as __fdiv_rn gives them.
+__device__ __forceinline__ float amax_over_6(float amax) {
+  return div_rn_mid(amax, 6.0f, 0.16666667163372039794921875f);   // RN(1/6)
+}
+__device__ __forceinline__ float scale_step(float sf, float gs) {
+  return (gs >= 1e-25f && gs <= 1e25f) ? div_rn_shared_rcp<false>(sf, gs, __frcp_rn(gs)) : __fdiv_rn(sf, gs);
 }
 
 // Quantises one block of 16 fp32 values, whose largest magnitude is `amax`, into 8 bytes of
@@ -114,11 +127,11 @@ __device__ __forceinline__ float div_rn_mid(float a, float b, float rb) {
 __device__ __forceinline__ void quantize_16_amax(const float* v, float amax, float gs, uint2& q8, uint32_t& sfb) {
   // divisions by 6 and by the group's gs: their reciprocals are constant or shared by the
   // thread's blocks, so the correctly rounded quotient takes three instructions
-  float s = __fmul_rn(div_rn_mid(amax, 6.0f, 0.16666667163372039794921875f), gs);   // RN(1/6)
+  float s = __fmul_rn(amax_over_6(amax), gs);
   s = fminf(fmaxf(s, 0.0f), 448.0f);
   sfb = (uint32_t)(uint8_t)__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3);
   const float sf = e4m3_to_float((uint8_t)sfb);
-  const float step = (gs >= 1e-25f && gs <= 1e25f) ? div_rn_shared_rcp<false>(sf, gs, __frcp_rn(gs)) : __fdiv_rn(sf, gs);
+  const float step = scale_step(sf, gs);
   // A dead block (step == 0) must yield x / 1 * 0 = +-0 with the sign of x, as the reference
   // computes: with divisor 1 and "reciprocal" 0 the shared-reciprocal division returns exactly
   // that (q = x * 0, remainder x, correction x * 0 + q), so no separate multiply is needed.
