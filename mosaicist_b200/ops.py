@@ -181,7 +181,13 @@ def to_mma_scale_layout(sf):
 def gemm_f16(a, b, out=None, max_ctas: int = 0):
     """C = A @ B for 2-D fp16 or bf16 CUDA tensors, A (m, k) and B (k, n) row-major (rows may be
     strided: a column slice of a wider matrix works as is), fp32 accumulation, output in the
-    input dtype.  The reference's dense problem (experiments/hopper_gemm/ref_cutedsl.py:50-74)."""
+    input dtype.  The reference's dense problem (experiments/hopper_gemm/ref_cutedsl.py:50-74).
+
+    The order of a row's sums depends on k and on whether there are more than 128 rows, and on nothing
+    else: with m <= 128 and k >= 4096 the contraction is summed as two halves, otherwise in one run.  So
+    a column shard has the bits of the whole product, and so have row blocks on one side of 128 rows; a
+    row computed in a batch of up to 128 and again in a larger one may differ in its last bit from
+    k = 4096 on."""
     return _host_ops.gemm_f16(a, b, out, max_ctas)
 
 
@@ -202,8 +208,8 @@ def mixed_grouped_gemm_int4(a, b_q, scales, group_offsets, group_rows, alpha=Non
     """bf16 activations x int4 weights (ports/hopper_mixed_dtype_grouped_gemm/problems.py:75-87).
 
     fused (default whenever k and group_size are multiples of 64): one kernel, converter warps
-    expand each stage of packed weights to bf16 in shared memory on their way to the tensor
-    core; the weights cross HBM once, as int4.  Otherwise two launches: expand the weights to
+    expand each stage of packed weights to bf16 in registers and put them into tensor memory as
+    the MMA's A operand; the weights cross HBM once, as int4.  Otherwise two launches: expand the weights to
     bf16 (`workspace`, (l, n, k) bf16, reusable while the weights do not change) and run the
     grouped bf16 GEMM.  Both produce the same bits."""
     return _host_ops.mixed_grouped_gemm_int4(a, b_q, scales, group_offsets, group_rows, alpha, group_size, workspace,

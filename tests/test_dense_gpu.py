@@ -126,3 +126,27 @@ def test_dense_split_forms_exact(m, n, k, tile_n, splits, dtype):
     assert ref.abs().max() <= 256                       # exact in bf16
     assert torch.equal(out[:, :n].double(), ref)
     assert torch.all(out[:, n:] == -7.0)
+
+
+@pytest.mark.parametrize("k", [1024, 4032, 4096, 7168])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_dense_rows_keep_their_bits_on_either_side_of_128(k, dtype):
+    """A row's bits do not depend on the batch it is computed in, as long as both batches have up to 128
+    rows or both have more; below k = 4096 not even that matters.  The two halves that batches of up to
+    128 rows are summed in from there on are no further from float64 than the single run."""
+    from mosaicist_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(k)
+    n = 1048
+    a = (torch.randn((600, k), device="cuda", generator=g) / k ** 0.5).to(dtype)
+    b = torch.randn((k, n), device="cuda", generator=g).to(dtype)
+    large = [ops.gemm_f16(a[:m], b)[:16] for m in (129, 256, 300, 600)]
+    small = [ops.gemm_f16(a[:m], b)[:16] for m in (16, 17, 64, 100, 128)] + [ops.gemm_f16(a[:16], b[:, :520].contiguous())]
+    small[-1] = torch.cat([small[-1], small[0][:, 520:]], 1)
+    assert all(torch.equal(x, large[0]) for x in large) and all(torch.equal(x, small[0]) for x in small)
+    if k < 4096:
+        assert torch.equal(small[0], large[0])
+        return
+    ref = a[:16].double() @ b.double()
+    # results are rounded to 16 bits: the sums' share of the error shows as a few per cent of it at most
+    assert (small[0].double() - ref).norm() <= 1.02 * (large[0].double() - ref).norm()
