@@ -276,8 +276,8 @@ int msc_grouped_gemm_bf16_ragged(const void* a, const void* b, const float* alph
                                  int l, int rows_total, int n, int k, int max_ctas, void* stream);
 /* The two calls above as one kernel (the reference's problem statement dequantises inside the
  * GEMM, problems.py:84-87): b_q (l, n, k/2) packed int4 and scales (l, n, k/group_size) bf16 are
- * read once; converter warps expand each 64-element K stage to bf16(q) * scale in shared memory
- * for the tensor core.  Same bits as the two-call path.  n % 256 == 0, k % 64 == 0,
+ * read once; converter warps expand each 128-element K stage to bf16(q) * scale in registers and
+ * put it into tensor memory, the weights being the MMA's A operand.  Same bits as the two-call path.  n % 256 == 0, k % 64 == 0,
  * group_size % 64 == 0 and dividing k (MSC_ERR_UNSUPPORTED otherwise). */
 int msc_grouped_gemm_bf16_int4_ragged(const void* a, const void* b_q, const void* scales,
                                       const float* alpha, const int32_t* group_offsets,
@@ -328,11 +328,13 @@ int msc_moe_plan_noalloc(const int32_t* ids, int entries, int expert_first, int 
  * and row_token (rows_cap) i32.  rows_cap is a multiple of 128 >= total_rows.  hidden % 64 == 0,
  * topk <= 64, a_q 16-byte aligned (rows leave shared memory as bulk copies).
  * sf_rows (rows_cap, hidden/16) u8 or NULL: staging for the scales.  With it (hidden % 256 == 0,
- * rows_cap a multiple of 128, both scale buffers 16-byte aligned) every row's scale bytes leave
- * as one bulk copy into sf_rows and a second kernel re-tiles them into a_sf - about 40 % less
- * time at top-8 than writing the tiling word by word; total_rows (device, i32, or NULL) is
- * the row count msc_moe_plan produced and bounds that pass, padding rows inside it receive
- * whatever sf_rows held.  Without it rows_cap and total_rows are ignored. */
+ * rows_cap a multiple of 128, both scale buffers 16-byte aligned) and tokens * topk > 4096 every
+ * row's scale bytes leave as one bulk copy into sf_rows and a second kernel re-tiles them into
+ * a_sf - about 40 % less time at 65536 rows than writing the tiling word by word; total_rows
+ * (device, i32, or NULL) is the row count msc_moe_plan produced and bounds that pass, padding
+ * rows inside it receive whatever sf_rows held.  For up to 4096 rows, where the second launch
+ * costs more than it saves, and without sf_rows the tiling is written directly: padding rows'
+ * scales stay as they were, sf_rows, rows_cap and total_rows are not used. */
 int msc_moe_permute_quantize(const void* tokens_bf16, const int32_t* ids, const float* weights,
                              const int32_t* rank, const int32_t* group_offsets,
                              const float* input_gs, int tokens, int hidden, int topk,

@@ -92,7 +92,8 @@ struct Int4Cursor {
   __device__ __forceinline__ int mma_n(int tt) const { return (tokens(tt) + GRAIN - 1) / GRAIN * GRAIN; }
 };
 
-// Eight nibbles of a word -> eight bf16 products with the scale, in K order.  The nibble with its
+// Eight nibbles of a word -> eight bf16 products with the scale, in K order.  The steps are those of
+// CUTLASS's int4 -> bf16 converter (cutlass/numeric_conversion.h, a published trick): the nibble with its
 // sign bit flipped is q + 8; put into the mantissa of 128.0 it reads 136 + q, and subtracting 136
 // is exact.  One byte permutation brings the two nibbles of a byte (one from the word, one from the
 // word shifted right by four) under one mask.

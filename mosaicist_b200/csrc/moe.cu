@@ -312,8 +312,9 @@ __global__ void __launch_bounds__(512) moe_permute_quantize_kernel(const Permute
 
 // ---- combine -----------------------------------------------------------------------------
 // One CTA per token (a few per token when there are not enough of them to fill the chip): the rows
-// holding the token's expert outputs are looked up once, then every thread sums 8 columns at a time over those rows, in the order of the token's pairs,
-// with the loads of up to eight rows issued before the first addition.
+// holding the token's expert outputs are looked up once, then every thread sums 8 columns at a time
+// over those rows, in the order of the token's pairs, with the loads of up to eight rows issued
+// before the first addition.
 __global__ void __launch_bounds__(256)
 moe_unpermute_kernel(const __nv_bfloat16* y, const int* ids,
                      const int* rank, const int* group_offsets,

@@ -222,8 +222,7 @@ int dt(const Tensor& x) { return x.scalar_type() == at::kBFloat16 ? 0 : 1; }
 
 // ---- the operators on tensors ------------------------------------------------------------------
 
-// Operands of a block-scaled GEMM over row-concatenated groups; elems: K-elements per operand byte
-// times 64, i.e. what one 512-byte scale chunk covers (NVFP4 64, MXFP8 128).
+// NVFP4 over padded batches: (l, m, k/2) by (l, n, k/2).
 Tensor gemm_masked(const Tensor& a_q, const Tensor& a_sf, const Tensor& b_q, const Tensor& b_sf,
                    const OptTensor& alpha, const OptTensor& masked_m, const msc_gemm_cfg& cfg, OptTensor out) {
   need(a_q, "a_q", kBytes);
@@ -247,6 +246,7 @@ Tensor gemm_masked(const Tensor& a_q, const Tensor& a_sf, const Tensor& b_q, con
   return *out;
 }
 
+// Row-concatenated groups, NVFP4 or MXFP8: `chunk` K-elements share a 512-byte piece of the scale tiling.
 Tensor gemm_ragged(bool mxfp8, const Tensor& a_q, const Tensor& a_sf, const Tensor& b_q, const Tensor& b_sf,
                    const Tensor& offsets, const Tensor& rows, const OptTensor& alpha, const OptTensor& row_scale,
                    msc_gemm_cfg cfg, OptTensor out) {

@@ -70,7 +70,7 @@ MAX_LAUNCHES = 5
 
 def section_of(kernel: str) -> str:
     """The part of the workload that launches `kernel`."""
-    for key, sec in (("dense_f16", "dense"), ("int4", "int4"), ("ep_", "ep"), ("moe_", "moe"), ("route_", "moe"),
+    for key, sec in (("dense", "dense"), ("int4", "int4"), ("ep_", "ep"), ("moe_", "moe"), ("route_", "moe"),
                      ("quantize", "quantize"), ("swizzle", "quantize"), ("amax", "quantize"), ("gemm_", "gemm")):
         if key in kernel:
             return sec
@@ -140,8 +140,11 @@ def run_workload(section: str = "all"):
         a = torch.randn((4096, 4096), device=dev, generator=g).half()
         b = torch.randn((4096, 4096), device=dev, generator=g).half()
         ops.gemm_f16(a, b)
+        # one tile per cluster: a weight matrix larger than L2 for a few rows, the contraction split
+        ops.gemm_f16(torch.randn((64, 8192), device=dev, generator=g).half(),
+                     torch.randn((8192, 10240), device=dev, generator=g).half())
 
-    # bf16 x int4 grouped GEMM (dequantise + bf16 grouped GEMM)
+    # bf16 x int4 grouped GEMM: groups of hundreds of rows (CTA pairs), then of a few rows
     rows = [256, 128, 384, 512, 128, 256, 256, 128]
     offs = np.concatenate([[0], np.cumsum(rows)[:-1]]).astype(np.int32)
     tot, nn, kk = int(sum(rows)), 2048, 7168
@@ -150,6 +153,10 @@ def run_workload(section: str = "all"):
         sc = (torch.randn((len(rows), nn, kk // 128), device=dev, generator=g) * 0.02).abs().bfloat16()
         ops.mixed_grouped_gemm_int4(x, u8(len(rows), nn, kk // 2), sc, torch.from_numpy(offs).to(dev),
                                     torch.tensor(rows, dtype=torch.int32, device=dev))
+        few = 16
+        ops.mixed_grouped_gemm_int4(x[:few * 128], u8(few, nn, kk // 2), sc[:1].expand(few, -1, -1).contiguous(),
+                                    torch.arange(few, dtype=torch.int32, device=dev) * 128,
+                                    torch.full((few,), 16, dtype=torch.int32, device=dev))
 
     # quantiser, SiLU*up quantiser, scale swizzle
     if want("quantize"):
