@@ -1,5 +1,6 @@
 // The row quantiser behind every stand-alone quantise entry point (NVFP4, NVFP4 of
-// SiLU(gate) * up, MXFP8): one kernel template over the output format and the input form.
+// SiLU(gate) * up, MXFP8): one kernel template over the output format, the input form and the layout
+// (masked batches or ragged groups).
 //
 // A thread owns 16 consecutive K-elements of FOUR rows, the rows 32 a + b (a = 0..3) of a
 // 128-row tile: in the 128-row MMA tiling the four scale words of those rows are 16 consecutive
@@ -7,13 +8,16 @@
 // (MXFP8) instead of 4-byte words 512 bytes apart, each of which costs an L2 transaction of its
 // own.  The loads of the four rows are issued before anything is computed; a warp reads 1 KB of
 // a row at a time.  Which rows are live is a property of the quad (its 128-row tile lies in one
-// ragged group, unless a group starts inside it) or of the row (masked batches), and the index arithmetic of the four blocks is
-// shared: multiplications by precomputed reciprocals instead of 64-bit divisions.
+// ragged group, unless a group starts inside it) or of the row (masked batches), and the index
+// arithmetic of the four blocks is shared: multiplications by precomputed reciprocals instead of
+// 64-bit divisions.
 //
 // Bound by HBM for MXFP8 and by a mix of issue slots and HBM for NVFP4.  Cold, 16384 x 7168,
 // against one thread per block with its own row search: MXFP8 bf16 99 -> 62 us (5.7 TB/s), ragged
 // groups 138 -> 62 us, fp32 106 -> 97 us; NVFP4 bf16 95 -> 71 us (4.3 TB/s), fp32 103 -> 97 us,
-// SiLU * up 132 -> 106 us.
+// SiLU * up 132 -> 106 us.  One kernel for both layouts, with the search of single rows inside it, cost
+// registers: 9 ragged groups of 666 rows, k 1920, 6.3 -> 6.7 us (6.3 with the search out of line and the
+// layouts apart).
 #pragma once
 
 #include "host_common.h"
