@@ -221,7 +221,8 @@ int msc_amax_global_scale(const void* x, int x_dtype, int l, long long elems_per
  *   x (rows, k) bf16 (x_dtype 0) or fp32 (1); q (rows, k) bytes; sf row-major (rows, k/32)
  *   (sf_layout 0) or in the MMA tiling (ceil(rows/128), k/128, 32, 16) (sf_layout 1), the form
  *   msc_grouped_gemm_mxfp8_ragged reads.  k % 128 == 0.
- * The ragged form quantises only rows inside a group (group_offsets ascending; the GEMMs want multiples of 128)
+ * The ragged form quantises only rows inside a group (group_offsets ascending; the GEMMs want
+ * multiples of 128)
  * and always writes tiled scales. */
 int msc_mxfp8_quantize(const void* x, int x_dtype, void* q, void* sf, int sf_layout, int rows, int k,
                        void* stream);
